@@ -98,18 +98,6 @@ struct Gather
     double weight[4];
 };
 
-// Unknowns of the coarsest direct solve: every cell with an open face except the first one,
-// which is pinned (the reference pins cell 0, PressureMultigrid.cpp:306-320; with no obstacle
-// the two are the same). Written by the rebuild, read by every V-cycle.
-struct CoarseInfo
-{
-    int n;       // unknowns
-    int pinned;  // pinned cell, -1 when no cell is open
-    int open;    // open cells (n + 1, or 0)
-    int map[64]; // cell -> unknown index, -1 for the pinned and the closed cells
-    int dirichlet; // Dirichlet air: unknowns only, nothing pinned, no mean and no gauge
-};
-
 struct LevelDesc
 {
     int w, h, S;
@@ -144,7 +132,6 @@ struct GridDesc
     int W, H, S;
     int levels;          // multigrid levels, the last one solved directly
     int tail;            // first level handled by the one-block coarse tail
-    int ncoarse;         // unknowns of the coarsest solve (cells - 1)
     double dx;
     LevelDesc lev[kMaxLevels];
     // fine-level vectors (padded layout)
@@ -158,9 +145,10 @@ struct GridDesc
     // face velocities, unpadded: u is (W+1) x H, v is W x (H+1), row-major
     void* u;
     void* v;
-    // coarsest inverse, up to ncoarse x ncoarse, row-major FP64, and its unknown map
+    // coarsest inverse, row-major FP64 (k_coarse_inverse), and the tail's layout and transfer tables
+    // (TailTable, fc_tail.cuh)
     double* coarse_inverse;
-    CoarseInfo* coarse;
+    const void* tail_table;
     SolveState* state;
     double4* partial;        // one slot per tile of the largest reduction
     unsigned int* counter;   // arrival counter of the reduction in flight

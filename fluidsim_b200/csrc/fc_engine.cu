@@ -11,6 +11,7 @@
 #include "fc_pcg.cuh"
 #include "fc_smooth.cuh"
 #include "fc_stage.cuh"
+#include "fc_tail.cuh"
 #include "fc_json.h"
 #include "fc_advect.cuh"
 #include "fc_tension.cuh"
@@ -161,6 +162,7 @@ struct HostLevel
     std::vector<Interp> px, py; // this level -> next
     std::vector<Gather> rx, ry; // next level's cells -> this level
     std::vector<unsigned char> rwx, rwy; // rx, ry as RestrictAxis<T> of the grid's precision
+    std::vector<unsigned char> pwx, pwy; // px, py as prolong_weights of the grid's precision
 };
 
 // Offset weights of a restriction table (what restrict_axis forms on the device).
@@ -179,6 +181,27 @@ template <typename T> std::vector<unsigned char> restrict_weights(const std::vec
                     r.mask |= 1u << p;
                 }
         out[c] = r;
+    }
+    return bytes;
+}
+
+// Prolongation weights on fixed coarse neighbours (the tail, fc_tail.cuh): fine cell f blends coarse cells
+// s = f / 2 - 1 + f % 2 and s + 1 (either may lie outside the level, clamped). The table's clamped
+// entries name s + 1 as their first cell with weight zero: that is weight one on the second.
+template <typename T> std::vector<unsigned char> prolong_weights(const std::vector<Interp>& table)
+{
+    std::vector<unsigned char> bytes(table.size() * sizeof(T));
+    T* out = reinterpret_cast<T*>(bytes.data());
+    for (size_t f = 0; f < table.size(); ++f)
+    {
+        const Interp& p = table[f];
+        const int s = int(f) / 2 - 1 + int(f) % 2;
+        if (p.first == s && (p.second == s + 1 || p.weight == 0.0))
+            out[f] = T(p.weight);
+        else if (p.first == s + 1 && p.weight == 0.0)
+            out[f] = T(1);
+        else
+            fail(FC_ERR_CUDA, "prolongation stencil outside coarse cells f / 2 - 1 .. f / 2 + 1");
     }
     return bytes;
 }
@@ -276,6 +299,7 @@ struct Grid
     std::vector<HostLevel> levels;
     int tail = 0;
     size_t tail_smem = 0;
+    int tail_threads = 0;
     int tail_cells = 1024; // largest level the one-CTA tail takes (autotuned)
 
     cudaStream_t stream = nullptr;
@@ -352,32 +376,85 @@ TileSizes tile_sizes(int precision, int shape)
     return tile_sizes_of<float, Tiling<float>::big, 8>();
 }
 
-// The coarse tail starts at the first level of at most g.tail_cells cells (and 1024 in FP64)
-// whose shared-memory footprint fits one CTA.
+// Layout of the grid's tail, with the arrays of its levels (null until the grid is allocated).
+TailTable tail_table(const Grid& g)
+{
+    TailTable t{};
+    t.first = g.tail;
+    t.smoothed = int(g.levels.size()) - 1 - g.tail;
+    for (int i = 0; i <= t.smoothed; ++i)
+    {
+        const HostLevel& L = g.levels[g.tail + i];
+        const LevelDesc& D = g.desc.lev[g.tail + i];
+        TailPlace& p = t.place[i];
+        p.w = L.w;
+        p.h = L.h;
+        p.S = L.S;
+        p.right = D.right;
+        p.down = D.down;
+        p.inv = D.inv;
+    }
+    t.rhs = g.tail == 0 ? g.desc.r : g.desc.lev[g.tail].rhs;
+    t.out = g.desc.lev[g.tail].sol;
+    tail_layout(t, g.elem == 4 ? kTailPlane<float> : kTailPlane<double>);
+    return t;
+}
+
+// The coarse tail starts at the first level of at most g.tail_cells cells (and 1024 in FP64, whose
+// strips take twice the registers) that the tail's register strips hold.
 void choose_tail(Grid& g)
 {
     const int limit_cells = g.elem == 4 ? g.tail_cells : std::min(g.tail_cells, 1024);
-    // Dynamic shared memory of the tail, within the 227 KB a CTA may hold beside its static
-    // shared memory (the register strips' edge rows: 19 KB in FP32, 36 KB in FP64).
-    const size_t limit_bytes = (g.elem == 4 ? 208 : 188) * 1024;
-    std::vector<int> w, h;
-    for (auto& l : g.levels)
-        w.push_back(l.w), h.push_back(l.h);
     const int n = int(g.levels.size());
+    g.tail = n - 1;
     for (int l = 0; l < n; ++l)
     {
-        const size_t bytes = tail_bytes(w.data(), h.data(), l, n, g.elem);
-        // The tail's register strips hold levels of up to kTailMaxSide x kTailMaxSide cells (the
-        // coarsest level, at most 64 cells, always fits).
-        if (w[l] * h[l] <= limit_cells && w[l] <= kTailMaxSide && h[l] <= kTailMaxSide && bytes <= limit_bytes)
+        // The tail's register strips hold levels of up to kTailMaxSide x kTailMaxSide cells and
+        // kTailMaxSmoothed of them (the coarsest level, at most 64 cells, always fits).
+        const HostLevel& L = g.levels[l];
+        if (L.w * L.h <= limit_cells && L.w <= kTailMaxSide && L.h <= kTailMaxSide && n - 1 - l <= kTailMaxSmoothed)
         {
             g.tail = l;
-            g.tail_smem = bytes;
-            return;
+            break;
         }
     }
-    g.tail = n - 1;
-    g.tail_smem = tail_bytes(w.data(), h.data(), n - 1, n, g.elem);
+    const TailTable t = tail_table(g);
+    int warps = 0;
+    for (int i = 0; i < t.smoothed; ++i)
+        warps += t.place[i].warps;
+    g.tail_smem = tail_bytes(t.elements, g.elem);
+    g.tail_threads = 32 * warps;
+    if (g.tail_smem > kTailMaxBytes || kTailHeader + t.tables * g.elem > kTailTableBytes ||
+        g.tail_threads > (g.elem == 4 ? kTailWideThreads : kTailThreads<double>))
+        fail(FC_ERR_CUDA, "coarse tail of a %dx%d grid does not fit one CTA", g.W, g.H);
+}
+
+// Uploads the tail's table (header and transfer weights) for the grid's current tail.
+void upload_tail_table(Grid& g)
+{
+    std::vector<unsigned char> bytes(kTailTableBytes, 0);
+    const TailTable t = tail_table(g);
+    std::memcpy(bytes.data(), &t, sizeof(t));
+    unsigned char* const tables = bytes.data() + kTailHeader;
+    for (int i = 0; i < t.smoothed; ++i)
+    {
+        const HostLevel& L = g.levels[g.tail + i];
+        const TailPlace& p = t.place[i];
+        // The first four values of a RestrictAxis are its weights.
+        auto axis = [&](const std::vector<unsigned char>& from, int at)
+        {
+            const size_t size = g.elem == 8 ? sizeof(RestrictAxis<double>) : sizeof(RestrictAxis<float>);
+            for (size_t c = 0; c < from.size() / size; ++c)
+                std::memcpy(tables + (at + 4 * c) * g.elem, from.data() + c * size, 4 * g.elem);
+        };
+        axis(L.rwy, p.rows);
+        axis(L.rwx, p.cols);
+        std::memcpy(tables + p.px * g.elem, L.pwx.data(), L.pwx.size());
+        std::memcpy(tables + p.py * g.elem, L.pwy.data(), L.pwy.size());
+    }
+    check(cudaMemcpyAsync(const_cast<void*>(g.desc.tail_table), bytes.data(), bytes.size(), cudaMemcpyHostToDevice, g.stream),
+        "tail table");
+    check(cudaStreamSynchronize(g.stream), "tail table"); // the host bytes must outlive the copy
 }
 
 // ------------------------------------------------------------------------------------------
@@ -495,8 +572,6 @@ size_t allocate_grid(Grid& g, bool allocate = true)
     d.dx = g.dx;
     d.levels = int(g.levels.size());
     d.tail = g.tail;
-    const HostLevel& last = g.levels.back();
-    d.ncoarse = last.w * last.h - 1;
     d.vec_tiles = ceil_div(W, kVecTileX) * ceil_div(H, kVecTileY);
     // The level-0 post kernel writes one (sum z, sum r z) pair per tile: slots for the most
     // tiles any region shape gives (two pairs to a double4 slot).
@@ -521,9 +596,8 @@ size_t allocate_grid(Grid& g, bool allocate = true)
     add((void**)&d.b, padded0 * sizeof(double));
     add(&d.u, g.faces_u * elem);
     add(&d.v, g.faces_v * elem);
-    // Up to every coarsest cell is an unknown (Dirichlet air pins none).
-    add((void**)&d.coarse_inverse, size_t(std::max(1, (d.ncoarse + 1) * (d.ncoarse + 1))) * sizeof(double));
-    add((void**)&d.coarse, sizeof(CoarseInfo));
+    add((void**)&d.coarse_inverse, kTailInverseBytes);
+    add(const_cast<void**>(&d.tail_table), kTailTableBytes);
     add((void**)&d.state, sizeof(SolveState));
     add((void**)&d.partial, size_t(std::max<long long>(std::max<long long>(d.vec_tiles, (post_pairs + 1) / 2), 1)) *
                                 sizeof(double4));
@@ -578,6 +652,8 @@ size_t allocate_grid(Grid& g, bool allocate = true)
             H.rwy = g.elem == 8 ? restrict_weights<double>(L.ry) : restrict_weights<float>(L.ry);
             add(&rwx[l], H.rwx.size());
             add(&rwy[l], H.rwy.size());
+            H.pwx = g.elem == 8 ? prolong_weights<double>(L.px) : prolong_weights<float>(L.px);
+            H.pwy = g.elem == 8 ? prolong_weights<double>(L.py) : prolong_weights<float>(L.py);
         }
     }
     // TMA maps: per level, kShapes region shapes, kMapsPerSet maps of 128 bytes.
@@ -622,6 +698,7 @@ size_t allocate_grid(Grid& g, bool allocate = true)
         }
     }
     d.solid = nullptr;
+    upload_tail_table(g);
     encode_stage_maps(g);
     check(cudaStreamSynchronize(g.stream), "grid set-up");
     return total;
@@ -954,6 +1031,7 @@ struct Plan
     int max_tail = 0;
     int padded_max[kMaxLevels] = {}; // largest padded level array of any grid, per level
     size_t tail_smem = 0;
+    int tail_threads = 0;
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;
     int graph_cap = -1;
@@ -1066,6 +1144,7 @@ std::unique_ptr<Plan> make_plan(const std::vector<Grid*>& grids, cudaStream_t st
         plan->max_levels = std::max(plan->max_levels, int(g->levels.size()));
         plan->max_tail = std::max(plan->max_tail, g->tail);
         plan->tail_smem = std::max(plan->tail_smem, g->tail_smem);
+        plan->tail_threads = std::max(plan->tail_threads, g->tail_threads);
         for (size_t l = 0; l < g->levels.size(); ++l)
             plan->padded_max[l] = std::max(plan->padded_max[l], g->levels[l].S * (g->levels[l].h + 2));
     }
@@ -1148,13 +1227,6 @@ template <typename T> void launch_rebuild(Plan& p)
     FC_LAUNCH_DEP(k_coefficients<T>, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec));
     for (int l = 0; l + 1 < p.max_levels; ++l)
         FC_LAUNCH_DEP(k_coarsen<T>, dim3(ceil_div(p.padded_max[l + 1], 256), p.n()), 256, 0, s, p.d_desc, l);
-    static const bool inverse_configured = [&]
-    {
-        check(cudaFuncSetAttribute(k_coarse_inverse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCoarseInverseSmem)),
-            "coarse inverse shared memory");
-        return true;
-    }();
-    (void)inverse_configured;
     if (p.precision == FC_PRECISION_MIXED)
         for (int l = 1; l < p.max_tail; ++l)
             FC_LAUNCH_DEP(k_weights_half, dim3(ceil_div(p.padded_max[l], 256), p.n()), 256, 0, s, p.d_desc, l);
@@ -1162,7 +1234,7 @@ template <typename T> void launch_rebuild(Plan& p)
     // level's inverse diagonal, and the coarsest factor from the level above it.
     for (int l = 0; l + 1 < p.max_levels; ++l)
         FC_LAUNCH_DEP(k_inverse_diagonal<T>, dim3(ceil_div(p.padded_max[l], 256), p.n()), 256, 0, s, p.d_desc, l);
-    FC_LAUNCH_DEP(k_coarse_inverse<T>, p.n(), kCoarseThreads, kCoarseInverseSmem, s, p.d_desc);
+    FC_LAUNCH_DEP(k_coarse_inverse<T>, p.n(), kCoarseThreads, 0, s, p.d_desc);
 }
 
 // Resident CTAs of the persistent smoothing kernels: two per SM in FP32, one in FP64 (their
@@ -1244,6 +1316,33 @@ template <typename T> void launch_smooth(Plan& p, int level, bool pre, bool depe
         : launch_smooth_shape<T, T, false>(p, r, level, shape, dependent, s);
 }
 
+// The coarse tail of every grid: one CTA each.
+template <typename T, int kThreads> void launch_tail_kernel(Plan& p, bool dependent, cudaStream_t s)
+{
+    auto kernel = k_mg_tail<T, kThreads>;
+    static const bool configured = [&]
+    {
+        check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTailMaxBytes)),
+            "tail shared memory");
+        return true;
+    }();
+    (void)configured;
+    if (dependent)
+        FC_LAUNCH_DEP(kernel, p.n(), kThreads, p.tail_smem, s, p.d_desc);
+    else
+        FC_LAUNCH(kernel, p.n(), kThreads, p.tail_smem, s, p.d_desc);
+}
+
+template <typename T> void launch_tail(Plan& p, bool dependent, cudaStream_t s)
+{
+    if constexpr (sizeof(T) == 4)
+    {
+        if (p.tail_threads > kTailThreads<T>)
+            return launch_tail_kernel<T, kTailWideThreads>(p, dependent, s);
+    }
+    launch_tail_kernel<T, kTailThreads<T>>(p, dependent, s);
+}
+
 // One application of the preconditioner to r: z, mean z, r.z and beta.
 template <typename T> void launch_precondition(Plan& p, bool use_mg)
 {
@@ -1255,7 +1354,7 @@ template <typename T> void launch_precondition(Plan& p, bool use_mg)
     }
     for (int l = 0; l < p.max_tail; ++l)
         launch_smooth<T>(p, l, true, true, s);
-    FC_LAUNCH_DEP(k_mg_tail<T>, p.n(), kTailThreads, p.tail_smem, s, p.d_desc);
+    launch_tail<T>(p, true, s);
     for (int l = p.max_tail - 1; l >= 0; --l)
         launch_smooth<T>(p, l, false, true, s);
 }
@@ -1268,22 +1367,6 @@ template <typename T> void launch_iteration(Plan& p, bool use_mg, int parity)
         p.at(p.vec), p.vec.count, parity);
     FC_LAUNCH_DEP(k_true_residual<T>, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec), 0);
     launch_precondition<T>(p, use_mg);
-}
-
-template <typename T> void set_kernel_attributes(Plan& p)
-{
-    // Always opted in: the tail's static edge rows count against the 48 KB default as well.
-    // The limit only ever rises (to the largest tail any plan has launched), so plans driven
-    // from several threads never lower it under one another's launches.
-    static std::mutex lock;
-    static size_t opted = 0;
-    std::lock_guard<std::mutex> guard(lock);
-    if (p.tail_smem > opted)
-    {
-        check(cudaFuncSetAttribute(k_mg_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(p.tail_smem)),
-            "tail shared memory");
-        opted = p.tail_smem;
-    }
 }
 
 // Projection set-up: states, right-hand side, warm start, first residual, first z.
@@ -1333,7 +1416,6 @@ template <typename T> void capture_projection(Plan& p, bool use_mg, int cap)
         cudaGraphDestroy(p.graph);
         p.graph = nullptr;
     }
-    set_kernel_attributes<T>(p);
     cudaStream_t s = p.stream;
     cudaGraph_t graph;
     check(cudaGraphCreate(&graph, 0), "graph create");
@@ -1401,7 +1483,6 @@ template <typename T> long long run_projection(Plan& p, bool use_mg, int max_ite
     const int cap = (std::max(max_iterations, 0) + 1) / 2 + 8;
     if (launch_mode.load() == FC_LAUNCH_STREAM)
     {
-        set_kernel_attributes<T>(p);
         const long long before = thread_launches;
         check(cudaMemcpyAsync(p.d_params, p.h_params, p.n() * sizeof(ProjectParams), cudaMemcpyHostToDevice, p.stream),
             "params");
@@ -2260,7 +2341,6 @@ void apply_preconditioner(Grid& g, const double* residual, double residual_mean,
     dispatch(g.precision, [&](auto zero)
     {
         using T = decltype(zero);
-        set_kernel_attributes<T>(p);
         FC_LAUNCH(k_pad_t<T>, blocks_for(g.cells), 256, 0, p.stream, g.staging, g.desc.r, g.W, g.H, g.S);
         launch_precondition<T>(p, use_mg);
         FC_LAUNCH(k_unpad_t<T>, blocks_for(g.cells), 256, 0, p.stream, g.desc.z, g.staging, g.W, g.H, g.S);
@@ -2292,7 +2372,6 @@ double time_kernel(Grid& g, int kernel, int repeats)
     dispatch(g.precision, [&](auto zero)
     {
         using T = decltype(zero);
-        set_kernel_attributes<T>(p);
         auto launch = [&]
         {
             switch (kernel)
@@ -2300,7 +2379,7 @@ double time_kernel(Grid& g, int kernel, int repeats)
             case 0: launch_smooth<T>(p, 0, true, false, p.stream); break;
             case 1: launch_smooth<T>(p, 0, false, false, p.stream); break;
             case 2: FC_LAUNCH(k_direction_operator<T>, p.vec.count, kVecThreads, 0, p.stream, p.d_desc, p.at(p.vec), 0); break;
-            default: FC_LAUNCH(k_mg_tail<T>, p.n(), kTailThreads, p.tail_smem, p.stream, p.d_desc); break;
+            default: launch_tail<T>(p, false, p.stream); break;
             }
         };
         launch(); // warm
@@ -2344,6 +2423,7 @@ void set_tail_cells(Grid& g, int cells)
     g.tail_cells = cells;
     choose_tail(g);
     g.desc.tail = g.tail;
+    upload_tail_table(g);
     g.plan.reset();
     g.coefficients_dirty = true; // mixed precision: FP16 copies of the newly smoothed levels
 }
@@ -2376,7 +2456,6 @@ double time_vcycles(Plan& p, int repeats)
             dispatch(p.precision, [&](auto zero)
             {
                 using T = decltype(zero);
-                set_kernel_attributes<T>(p);
                 launch_precondition<T>(p, true);
             });
         };

@@ -43,6 +43,30 @@ def test_vcycle_matches_restatement_at_every_tail_threshold(oracle, size, cells)
     assert np.abs(z - expected).max() <= 1e-10 * scale
 
 
+# Around the widths at which a level's row groups take 8, 16 and 32 lanes, heights that fill the last
+# group of a warp or leave it short, and grids whose tail is the coarsest level alone.
+GROUPS = [(16, 64), (17, 16), (32, 32), (33, 31), (31, 33), (34, 5), (64, 17), (15, 66), (8, 8), (9, 7), (1, 1), (66, 50)]
+
+
+@pytest.mark.parametrize("precision,bound", [("fp64", 1e-10), ("fp32", 5e-4)])
+@pytest.mark.parametrize("size", GROUPS, ids=lambda s: f"{s[0]}x{s[1]}")
+def test_vcycle_matches_restatement_at_row_group_edges(oracle, size, precision, bound):
+    """The bounds are those of the tests beside this one."""
+    w, h = size
+    density, residual = _case(w, h)
+    inv_u, inv_v, _ = oracle.coefficients(density)
+    mg = oracle.Multigrid(w, h)
+    assert mg.rebuild(inv_u, inv_v)
+    expected = mg.apply(residual)
+    s = scenes.Scene(w, h, 1.0, 1.0, 1.0, 1.0, np.ones((h, w)), np.zeros((h, w + 1)), np.zeros((h + 1, w)),
+                     liquid_mass=[density], gas_mass=[np.zeros((h, w))])
+    g = FluidGrid(w, h, 1.0, precision)
+    scenes.upload_scene(g, s)
+    g.setTailCells(4096)
+    z = g.applyPreconditioner(residual)
+    assert np.abs(z - expected).max() <= bound * max(1.0, np.abs(expected).max())
+
+
 @pytest.mark.parametrize("size", [(64, 64), (190, 130), (1000, 3)], ids=lambda s: f"{s[0]}x{s[1]}")
 def test_fp32_tail_stays_close_to_fp64(size):
     """The FP32 tail differs from the FP64 one only by rounding."""
