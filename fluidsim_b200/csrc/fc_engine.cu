@@ -1961,6 +1961,7 @@ struct ViscWork
     double4* partial;
     unsigned int* counter;
     double2* comp;
+    size_t tail = 0; // first level of the one-CTA tail
 };
 
 // Lays out (and with allocate, allocates) the viscosity workspace of a grid.
@@ -1991,7 +1992,7 @@ size_t viscosity_layout(const Grid& g, ViscWork* work, char* base)
         v.x = take(nodes * 2 * e);
         v.next = take(nodes * 2 * e);
         v.rhs = take(nodes * 2 * e);
-        v.res = take(nodes * 2 * e);
+        v.half = take(nodes * 2 * e);
         if (work)
             work->lev[l] = v;
     }
@@ -2022,6 +2023,22 @@ size_t viscosity_layout(const Grid& g, ViscWork* work, char* base)
     return total;
 }
 
+// First level of the one-CTA tail: the first whose levels fit 200 KB of shared memory together (in
+// FP32 4,300 nodes, so a first level of up to 3,200, e.g. 56 x 56). At 4096 x 4096 it takes the levels
+// from 32 x 32 on.
+size_t viscosity_tail(const ViscWork& w, size_t elem)
+{
+    size_t first = w.lev.size() - 1, bytes = 0;
+    for (size_t l = w.lev.size(); l-- > 0;)
+    {
+        bytes += visc_tail_bytes((w.lev[l].w + 1) * (w.lev[l].h + 1), elem);
+        if (bytes > kViscTailMaxBytes || w.lev.size() - l > size_t(kViscTailLevels))
+            break;
+        first = l;
+    }
+    return first;
+}
+
 ViscWork viscosity_workspace(Grid& g, cudaStream_t s)
 {
     const size_t bytes = viscosity_layout(g, nullptr, nullptr);
@@ -2036,38 +2053,56 @@ ViscWork viscosity_workspace(Grid& g, cudaStream_t s)
     }
     ViscWork w;
     viscosity_layout(g, &w, g.visc_arena);
+    w.tail = viscosity_tail(w, g.elem);
     return w;
 }
 
-template <typename T> void viscosity_cycle(ViscWork& w, size_t l, void* b, double dt, const unsigned char* solid,
-    cudaStream_t s)
+template <typename T> void launch_viscosity_tail(ViscWork& w, size_t l, double dt, cudaStream_t s)
+{
+    static const bool configured = [&]
+    {
+        check(cudaFuncSetAttribute(k_visc_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kViscTailMaxBytes)),
+            "viscosity tail shared memory");
+        return true;
+    }();
+    (void)configured;
+    ViscTail t{};
+    int nodes = 0;
+    for (size_t k = l; k < w.lev.size(); ++k)
+    {
+        t.lev[t.levels++] = w.lev[k];
+        nodes += (w.lev[k].w + 1) * (w.lev[k].h + 1);
+    }
+    FC_LAUNCH_DEP(k_visc_tail<T>, 1, kViscTailThreads, visc_tail_bytes(nodes, sizeof(T)), s, t, dt, w.state);
+}
+
+// One V-cycle of level l on b, from the sweep from zero that b's writer left in L.x (below the tail's
+// first level the tail does it all).
+template <typename T> void viscosity_cycle(ViscWork& w, size_t l, void* b, double dt, cudaStream_t s)
 {
     ViscLevel& L = w.lev[l];
-    const unsigned char* mask = l == 0 ? solid : nullptr;
-    const int blocks = ceil_div((L.w + 1) * (L.h + 1), kViscThreads);
-    if (l + 1 == w.lev.size())
+    if (l == w.tail)
     {
-        ViscLevel c = L;
-        c.rhs = b;
-        FC_LAUNCH_DEP(k_visc_coarse<T>, 1, kViscCoarseNodes, 0, s, c, dt, mask, w.state);
+        const void* saved = L.rhs;
+        L.rhs = b;
+        launch_viscosity_tail<T>(w, l, dt, s);
+        L.rhs = const_cast<void*>(saved);
         return;
     }
-    auto smooth = [&](int zero)
+    const int blocks = ceil_div((L.w + 1) * (L.h + 1), kViscThreads);
+    auto tiles = [](const ViscLevel& v) { return dim3(ceil_div(v.w + 1, kViscTileX), ceil_div(v.h + 1, kViscTileY)); };
+    auto smooth = [&]
     {
-        FC_LAUNCH_DEP(k_visc_smooth<T>, blocks, kViscThreads, 0, s, L, dt, mask, b, zero, w.state);
+        FC_LAUNCH_DEP(k_visc_smooth<T>, blocks, kViscThreads, 0, s, L, dt, b, w.state);
         std::swap(L.x, L.next);
     };
-    smooth(1);
-    smooth(0);
-    FC_LAUNCH_DEP((k_visc_residual<T, kResidualPlain>), blocks, kViscThreads, 0, s, L, dt, mask, L.x, b, L.res, w.state,
-        w.partial, w.counter, 0.0);
+    smooth();
     ViscLevel& C = w.lev[l + 1];
-    FC_LAUNCH_DEP(k_visc_restrict<T>, ceil_div((C.w + 1) * (C.h + 1), kViscThreads), kViscThreads, 0, s, L, C, w.state);
-    viscosity_cycle<T>(w, l + 1, C.rhs, dt, solid, s);
-    FC_LAUNCH_DEP(k_visc_prolong<T>, blocks, kViscThreads, 0, s, L, C, mask, w.state);
+    FC_LAUNCH_DEP(k_visc_restrict<T>, tiles(C), kViscThreads, 0, s, L, C, dt, b, l + 1 < w.tail ? 1 : 0, w.state);
+    viscosity_cycle<T>(w, l + 1, C.rhs, dt, s);
+    FC_LAUNCH_DEP(k_visc_prolong_smooth<T>, tiles(L), kViscThreads, 0, s, L, C, dt, b, w.state);
     std::swap(L.x, L.next);
-    smooth(0);
-    smooth(0);
+    smooth();
 }
 
 struct ViscResult
@@ -2108,12 +2143,18 @@ template <typename T> ViscResult viscosity_solve(Grid& g, double dt, double tole
             L.material, L.w, L.h, L.dx, const_cast<void*>(L.coeff));
     }
     const unsigned char* solid = g.has_solid ? g.solid : nullptr;
+    for (size_t l = 0; l < w.lev.size(); ++l)
+    {
+        const ViscLevel& L = w.lev[l];
+        FC_LAUNCH(k_visc_diagonal<T>, ceil_div((L.w + 1) * (L.h + 1), kViscThreads), kViscThreads, 0, s, L, dt,
+            l == 0 ? solid : nullptr, const_cast<void*>(L.half));
+    }
     const int nodes = (g.W + 1) * (g.H + 1);
     const int blocks = ceil_div(nodes, kViscThreads);
     const int reduce_blocks = ceil_div(nodes, kViscThreads * kViscReduceNodes);
     ViscLevel& L0 = w.lev[0];
     FC_LAUNCH(k_visc_pack<T>, blocks, kViscThreads, 0, s, g.W, g.H, g.desc.u, g.desc.v, L0.coeff, solid, w.solution, w.rhs);
-    FC_LAUNCH((k_visc_residual<T, kResidualInitial>), reduce_blocks, kViscThreads, 0, s, L0, dt, solid, w.solution, w.rhs,
+    FC_LAUNCH((k_visc_residual<T, kResidualInitial>), reduce_blocks, kViscThreads, 0, s, L0, dt, w.solution, w.rhs,
         w.residual, w.state, w.partial, w.counter, tolerance);
     ViscState h{};
     auto read_state = [&]
@@ -2134,17 +2175,16 @@ template <typename T> ViscResult viscosity_solve(Grid& g, double dt, double tole
         const int batch = max_iterations < 0 ? 4 : std::min(4, max_iterations - result.iterations);
         for (int i = 0; i < batch; ++i)
         {
-            viscosity_cycle<T>(w, 0, w.residual, dt, solid, s);
+            viscosity_cycle<T>(w, 0, w.residual, dt, s);
             FC_LAUNCH_DEP(k_visc_dot_rz<T>, reduce_blocks, kViscThreads, 0, s, nodes, L0.coeff, w.residual, L0.x, w.state,
                 w.partial, w.counter);
             FC_LAUNCH_DEP(k_visc_direction<T>, blocks, kViscThreads, 0, s, nodes, L0.x, w.direction, w.state);
-            FC_LAUNCH_DEP((k_visc_apply<T, true>), reduce_blocks, kViscThreads, 0, s, L0, dt, solid, w.direction, w.product,
-                w.state, w.partial, w.counter);
+            FC_LAUNCH_DEP(k_visc_apply<T>, reduce_blocks, kViscThreads, 0, s, L0, dt, w.direction, w.product, w.state, w.partial, w.counter);
             FC_LAUNCH_DEP(k_visc_update<T>, blocks, kViscThreads, 0, s, nodes, w.solution, w.residual, w.direction,
-                w.product, w.state);
+                w.product, L0.half, L0.x, w.state);
         }
         result.iterations += batch;
-        FC_LAUNCH_DEP((k_visc_residual<T, kResidualTruth>), reduce_blocks, kViscThreads, 0, s, L0, dt, solid, w.solution, w.rhs,
+        FC_LAUNCH_DEP((k_visc_residual<T, kResidualTruth>), reduce_blocks, kViscThreads, 0, s, L0, dt, w.solution, w.rhs,
             w.truth, w.state, w.partial, w.counter, tolerance);
         read_state();
         result.relative_residual = std::sqrt(h.truth / std::max(h.energy, 1e-30));
@@ -2153,7 +2193,8 @@ template <typename T> ViscResult viscosity_solve(Grid& g, double dt, double tole
         if (h.truth <= h.target)
             break;
         if (h.stopped)
-            FC_LAUNCH_DEP(k_visc_refresh<T>, blocks, kViscThreads, 0, s, nodes, w.truth, w.residual, w.state);
+            FC_LAUNCH_DEP(k_visc_refresh<T>, blocks, kViscThreads, 0, s, nodes, w.truth, w.residual, L0.half, L0.x,
+                w.state);
     }
     FC_LAUNCH(k_visc_unpack<T>, blocks, kViscThreads, 0, s, g.W, g.H, w.solution, g.desc.u, g.desc.v);
     check(cudaStreamSynchronize(s), "viscosity");

@@ -7,6 +7,14 @@
 // CG recurrences and 4-iteration true-residual check. Vectors are in the working precision;
 // every reduction and CG scalar is FP64.
 //
+// A pass is bound by instructions and launches more than by bytes (206 instructions a node and 41 %
+// of DRAM peak in a sweep that formed its diagonal and mask; 2.5 to 3 us for a pass of a small
+// level), so the V-cycle takes few of them: the sweep from zero is written by whatever writes its
+// right-hand side, the residual is restricted where it is formed (k_visc_restrict), the prolongation
+// is swept where it is formed (k_visc_prolong_smooth), and the small levels run in one CTA
+// (k_visc_tail): 17 launches a CG iteration instead of 41 at 321 x 239. Measured, whole solves in
+// FP32 before and after: 321 x 239 6.65 -> 5.69 ms, 4096 x 4096 189 -> 159 ms.
+//
 // Layout: the (w+1) x (h+1) node lattice of a level, row-major; node p holds u face p (x) and v
 // face p (y) as one 2-vector, and 4 coefficients (cell mu, vertex mu, u-face mass, v-face mass).
 // Reads outside a field clamp to its edge, as the reference's field accessor does. One thread
@@ -21,7 +29,6 @@ namespace fc
 {
 
 constexpr int kViscThreads = 256;
-constexpr int kViscCoarseNodes = 256; // the coarsest level fits one block
 // Nodes per thread of the kernels that end in a grid reduction: a block covers this many runs
 // of kViscThreads consecutive nodes, so the per-block reduction, fence and atomic are paid a
 // quarter as often.
@@ -60,10 +67,10 @@ struct ViscLevel
     double dx;
     const void* material; // 2 per cell (density, viscosity)
     const void* coeff;    // 4 per node
+    const void* half;     // 2 per node: half the inverse diagonal, zero where there is no open face
     void* x;
     void* next;
     void* rhs;
-    void* res;
 };
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
@@ -77,16 +84,6 @@ __device__ __forceinline__ bool solid_at(const unsigned char* solid, int w, int 
 {
     return solid && solid[(long long)y * w + x];
 }
-
-template <typename T> struct Nodes
-{
-    using T2 = typename Vec<T>::two;
-    using T4 = typename Vec<T>::four;
-    int w, h;
-    __device__ long long at(int x, int y) const { return (long long)clampi(y, 0, h) * (w + 1) + clampi(x, 0, w); }
-    __device__ T2 load(const void* f, int x, int y) const { return static_cast<const T2*>(f)[at(x, y)]; }
-    __device__ T4 coeff(const void* c, int x, int y) const { return static_cast<const T4*>(c)[at(x, y)]; }
-};
 
 // Deterministic two-level reduction. Blocks arrive in fixed groups of NT consecutive blocks:
 // the last block of a group to arrive folds the group's partials (one per thread, then
@@ -240,33 +237,36 @@ __global__ void k_visc_coefficients(const void* material, int w, int h, double d
 // Operator (ViscosityKernels.h:8-75)
 // ---------------------------------------------------------------------------------------------
 
-template <typename T>
-__device__ __forceinline__ T shear_term(const Nodes<T>& L, const void* f, const void* c, int x, int y)
+// Offsets of a node and its neighbours in a row-major lattice, with the reference's clamps: left,
+// right, up, down, and the two diagonal ones that the shear terms read.
+struct Around
 {
-    const auto p = L.load(f, x, y);
-    return L.coeff(c, x, y).y * ((p.x - L.load(f, x, y - 1).x) + (p.y - L.load(f, x - 1, y).y));
+    int own, left, right, up, down, down_left, up_right;
+};
+
+__device__ __forceinline__ Around around(int w, int h, int x, int y)
+{
+    const int row = y * (w + 1), above = max(y - 1, 0) * (w + 1), below = min(y + 1, h) * (w + 1);
+    const int left = max(x - 1, 0), right = min(x + 1, w);
+    return {row + x, row + left, row + right, above + x, below + x, below + left, above + right};
 }
 
-// mass f(p) + dt stress(f)(p) for both components of node p, before the valid-face mask.
+// mass f + dt stress(f) for both components of a node, before the valid-face mask: f at the offsets
+// n, the coefficients at the offsets m.
 template <typename T>
-__device__ __forceinline__ void operator_at(const Nodes<T>& L, const void* f, const void* coeff, T dt, int x, int y,
-    T& ax, T& ay)
+__device__ __forceinline__ void operator_at(const typename Vec<T>::two* f, const Around& n, const typename Vec<T>::four* coeff,
+    const Around& m, T dt, T& ax, T& ay)
 {
-    const auto c = L.load(f, x, y);
-    const auto a = L.coeff(coeff, x, y);
-    const T t = shear_term<T>(L, f, coeff, x, y);
-    const T nx = T(2) * (L.coeff(coeff, x - 1, y).x * (c.x - L.load(f, x - 1, y).x) + a.x * (c.x - L.load(f, x + 1, y).x));
-    const T ny = T(2) * (L.coeff(coeff, x, y - 1).x * (c.y - L.load(f, x, y - 1).y) + a.x * (c.y - L.load(f, x, y + 1).y));
-    ax = a.z * c.x + dt * (nx + (t - shear_term<T>(L, f, coeff, x, y + 1)));
-    ay = a.w * c.y + dt * (ny + (t - shear_term<T>(L, f, coeff, x + 1, y)));
-}
-
-template <typename T>
-__device__ __forceinline__ void diagonal_at(const Nodes<T>& L, const void* coeff, T dt, int x, int y, T& dx_, T& dy_)
-{
-    const auto c = L.coeff(coeff, x, y);
-    dx_ = c.z + dt * (T(2) * (c.x + L.coeff(coeff, x - 1, y).x) + c.y + L.coeff(coeff, x, y + 1).y);
-    dy_ = c.w + dt * (T(2) * (c.x + L.coeff(coeff, x, y - 1).x) + c.y + L.coeff(coeff, x + 1, y).y);
+    const auto c = f[n.own], fl = f[n.left], fr = f[n.right], fu = f[n.up], fd = f[n.down];
+    const T down_left = f[n.down_left].y, up_right = f[n.up_right].x;
+    const auto a = coeff[m.own];
+    const T t = a.y * ((c.x - fu.x) + (c.y - fl.y));
+    const T below = coeff[m.down].y * ((fd.x - c.x) + (fd.y - down_left));
+    const T beside = coeff[m.right].y * ((fr.x - up_right) + (fr.y - c.y));
+    const T nx = T(2) * (coeff[m.left].x * (c.x - fl.x) + a.x * (c.x - fr.x));
+    const T ny = T(2) * (coeff[m.up].x * (c.y - fu.y) + a.x * (c.y - fd.y));
+    ax = a.z * c.x + dt * (nx + (t - below));
+    ay = a.w * c.y + dt * (ny + (t - beside));
 }
 
 struct FaceMask
@@ -287,47 +287,59 @@ __device__ __forceinline__ FaceMask face_mask(int w, int h, int x, int y, const 
     return m;
 }
 
+// Half the inverse diagonal of a level's operator, once per solve: the damped Jacobi sweep is then a
+// multiplication (the two divisions and the face mask were a quarter of its instructions).
+template <typename T>
+__global__ void __launch_bounds__(kViscThreads) k_visc_diagonal(ViscLevel lv, double dt, const unsigned char* solid, void* half)
+{
+    using T2 = typename Vec<T>::two;
+    using T4 = typename Vec<T>::four;
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= (lv.w + 1) * (lv.h + 1))
+        return;
+    const int x = n % (lv.w + 1), y = n / (lv.w + 1);
+    const FaceMask m = face_mask(lv.w, lv.h, x, y, solid);
+    const Around o = around(lv.w, lv.h, x, y);
+    const T4* coeff = static_cast<const T4*>(lv.coeff);
+    const T4 c = coeff[o.own];
+    const T dx = c.z + T(dt) * (T(2) * (c.x + coeff[o.left].x) + c.y + coeff[o.down].y);
+    const T dy = c.w + T(dt) * (T(2) * (c.x + coeff[o.up].x) + c.y + coeff[o.right].y);
+    static_cast<T2*>(half)[n] = T2{m.u ? T(0.5) / dx : T(0), m.v ? T(0.5) / dy : T(0)};
+}
+
 __device__ __forceinline__ bool visc_stopped(const ViscState* s) { return s->stopped || s->breakdown; }
 
-// out = A f on valid faces (ViscosityKernels.h "apply"); with dq, also d.Ad reduced into the CG
-// step length alpha (ViscosityKernels.h "scalar" mode 2).
-template <typename T, bool kDot>
-__global__ void __launch_bounds__(kViscThreads) k_visc_apply(ViscLevel lv, double dt, const unsigned char* solid,
-    const void* f, void* out, ViscState* state, double4* partial, unsigned int* counter)
+// out = A f on valid faces (ViscosityKernels.h "apply"), and d.Ad reduced into the CG step length
+// alpha (ViscosityKernels.h "scalar" mode 2).
+template <typename T>
+__global__ void __launch_bounds__(kViscThreads) k_visc_apply(ViscLevel lv, double dt, const void* f, void* out,
+    ViscState* state, double4* partial, unsigned int* counter)
 {
     allow_dependents();
     dependency_wait();
     using T2 = typename Vec<T>::two;
-    constexpr int kNodes = kDot ? kViscReduceNodes : 1;
-    const Nodes<T> L{lv.w, lv.h};
+    using T4 = typename Vec<T>::four;
     const bool stopped = visc_stopped(state);
     double dq = 0.0;
 #pragma unroll 1
-    for (int k = 0; k < kNodes; ++k)
+    for (int k = 0; k < kViscReduceNodes && !stopped; ++k)
     {
-        const int n = (blockIdx.x * kNodes + k) * blockDim.x + threadIdx.x;
+        const int n = (blockIdx.x * kViscReduceNodes + k) * blockDim.x + threadIdx.x;
         if (n >= (lv.w + 1) * (lv.h + 1))
             break;
-        const int x = n % (lv.w + 1), y = n / (lv.w + 1);
+        const Around o = around(lv.w, lv.h, n % (lv.w + 1), n / (lv.w + 1));
+        const T2 half = static_cast<const T2*>(lv.half)[n];
+        T ax, ay;
+        operator_at<T>(static_cast<const T2*>(f), o, static_cast<const T4*>(lv.coeff), o, T(dt), ax, ay);
         T2 r;
-        r.x = r.y = T(0);
-        if (!stopped)
-        {
-            const FaceMask m = face_mask(lv.w, lv.h, x, y, solid);
-            T ax, ay;
-            operator_at<T>(L, f, lv.coeff, T(dt), x, y, ax, ay);
-            r.x = m.u ? ax : T(0);
-            r.y = m.v ? ay : T(0);
-            const T2 d = static_cast<const T2*>(f)[n];
-            dq += double(d.x) * double(r.x) + double(d.y) * double(r.y);
-        }
+        r.x = half.x != T(0) ? ax : T(0);
+        r.y = half.y != T(0) ? ay : T(0);
+        const T2 d = static_cast<const T2*>(f)[n];
+        dq += double(d.x) * double(r.x) + double(d.y) * double(r.y);
         static_cast<T2*>(out)[n] = r;
     }
-    if (!kDot)
-        return;
     double4 total;
-    const int blocks = gridDim.x;
-    if (visc_arrive_last<kViscThreads>(partial, counter, blockIdx.x, blocks,
+    if (visc_arrive_last<kViscThreads>(partial, counter, blockIdx.x, gridDim.x,
             block_reduce4<kViscThreads>(make_double4(dq, 0, 0, 0), 0), &total, 0))
     {
         if (threadIdx.x == 0 && !stopped)
@@ -343,104 +355,79 @@ __global__ void __launch_bounds__(kViscThreads) k_visc_apply(ViscLevel lv, doubl
     }
 }
 
-// Damped Jacobi (ViscosityKernels.h "smooth"): x + (b - A x) / (2 D), or b / (2 D) from zero.
+// Damped Jacobi (ViscosityKernels.h "smooth"): x + (b - A x) / (2 D). The sweep from zero, b / (2 D),
+// has no kernel: whatever writes b writes it to x as well.
 template <typename T>
-__global__ void __launch_bounds__(kViscThreads) k_visc_smooth(ViscLevel lv, double dt, const unsigned char* solid,
-    const void* b, int zero, const ViscState* state)
+__device__ __forceinline__ typename Vec<T>::two jacobi(const typename Vec<T>::two& c, const typename Vec<T>::two& b,
+    const typename Vec<T>::two& half, T ax, T ay)
+{
+    typename Vec<T>::two out;
+    out.x = half.x != T(0) ? c.x + (b.x - ax) * half.x : T(0);
+    out.y = half.y != T(0) ? c.y + (b.y - ay) * half.y : T(0);
+    return out;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kViscThreads) k_visc_smooth(ViscLevel lv, double dt, const void* b, const ViscState* state)
 {
     allow_dependents();
     dependency_wait();
     using T2 = typename Vec<T>::two;
-    const Nodes<T> L{lv.w, lv.h};
+    using T4 = typename Vec<T>::four;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= (lv.w + 1) * (lv.h + 1))
+    if (n >= (lv.w + 1) * (lv.h + 1) || visc_stopped(state))
         return;
-    const int x = n % (lv.w + 1), y = n / (lv.w + 1);
-    T2 out;
-    out.x = out.y = T(0);
-    if (!visc_stopped(state))
-    {
-        const FaceMask m = face_mask(lv.w, lv.h, x, y, solid);
-        T dxx, dyy;
-        diagonal_at<T>(L, lv.coeff, T(dt), x, y, dxx, dyy);
-        const T2 bb = static_cast<const T2*>(b)[n];
-        T vx, vy;
-        if (zero)
-        {
-            vx = T(0.5) * bb.x / dxx;
-            vy = T(0.5) * bb.y / dyy;
-        }
-        else
-        {
-            T ax, ay;
-            operator_at<T>(L, lv.x, lv.coeff, T(dt), x, y, ax, ay);
-            const T2 c = static_cast<const T2*>(lv.x)[n];
-            vx = c.x + T(0.5) * (bb.x - ax) / dxx;
-            vy = c.y + T(0.5) * (bb.y - ay) / dyy;
-        }
-        out.x = m.u ? vx : T(0);
-        out.y = m.v ? vy : T(0);
-    }
-    static_cast<T2*>(lv.next)[n] = out;
+    const Around o = around(lv.w, lv.h, n % (lv.w + 1), n / (lv.w + 1));
+    const T2* x = static_cast<const T2*>(lv.x);
+    T ax, ay;
+    operator_at<T>(x, o, static_cast<const T4*>(lv.coeff), o, T(dt), ax, ay);
+    static_cast<T2*>(lv.next)[n] =
+        jacobi<T>(x[n], static_cast<const T2*>(b)[n], static_cast<const T2*>(lv.half)[n], ax, ay);
 }
 
-// Statistics a residual pass can reduce (ViscosityKernels.h "first_reduce" modes 0 and 3).
+// Statistics a residual pass reduces (ViscosityKernels.h "first_reduce" modes 0 and 3).
 enum ViscResidualMode
 {
-    kResidualPlain = 0,   // multigrid residual, no reduction
     kResidualInitial = 1, // |r|^2_M, |x|^2_M, total mass; sets the target
     kResidualTruth = 2    // |r|^2_M into state->truth
 };
 
-// out = b - A f on valid faces.
+// out = b - A f on valid faces; the initial one also starts the V-cycle's sweep from zero (lv.x).
 template <typename T, int kMode>
-__global__ void __launch_bounds__(kViscThreads) k_visc_residual(ViscLevel lv, double dt, const unsigned char* solid,
-    const void* f, const void* b, void* out, ViscState* state, double4* partial, unsigned int* counter,
-    double tolerance)
+__global__ void __launch_bounds__(kViscThreads) k_visc_residual(ViscLevel lv, double dt, const void* f, const void* b,
+    void* out, ViscState* state, double4* partial, unsigned int* counter, double tolerance)
 {
     allow_dependents();
     dependency_wait();
     using T2 = typename Vec<T>::two;
-    constexpr int kNodes = kMode == kResidualPlain ? 1 : kViscReduceNodes;
-    const Nodes<T> L{lv.w, lv.h};
-    if (kMode == kResidualPlain && visc_stopped(state))
-    {
-        const int n = blockIdx.x * blockDim.x + threadIdx.x;
-        if (n < (lv.w + 1) * (lv.h + 1))
-            static_cast<T2*>(out)[n] = T2{T(0), T(0)};
-        return;
-    }
+    using T4 = typename Vec<T>::four;
     double4 mine = make_double4(0, 0, 0, 0);
 #pragma unroll 1
-    for (int k = 0; k < kNodes; ++k)
+    for (int k = 0; k < kViscReduceNodes; ++k)
     {
-        const int n = (blockIdx.x * kNodes + k) * blockDim.x + threadIdx.x;
+        const int n = (blockIdx.x * kViscReduceNodes + k) * blockDim.x + threadIdx.x;
         if (n >= (lv.w + 1) * (lv.h + 1))
             break;
-        const int x = n % (lv.w + 1), y = n / (lv.w + 1);
-        const FaceMask m = face_mask(lv.w, lv.h, x, y, solid);
+        const Around o = around(lv.w, lv.h, n % (lv.w + 1), n / (lv.w + 1));
+        const T2 half = static_cast<const T2*>(lv.half)[n];
         T ax, ay;
-        operator_at<T>(L, f, lv.coeff, T(dt), x, y, ax, ay);
+        operator_at<T>(static_cast<const T2*>(f), o, static_cast<const T4*>(lv.coeff), o, T(dt), ax, ay);
         const T2 bb = static_cast<const T2*>(b)[n];
         T2 r;
-        r.x = m.u ? bb.x - ax : T(0);
-        r.y = m.v ? bb.y - ay : T(0);
+        r.x = half.x != T(0) ? bb.x - ax : T(0);
+        r.y = half.y != T(0) ? bb.y - ay : T(0);
         static_cast<T2*>(out)[n] = r;
-        if (kMode != kResidualPlain)
+        const T4 c = static_cast<const T4*>(lv.coeff)[n];
+        const double rx = r.x, ry = r.y;
+        mine.x += rx / double(c.z) * rx + ry / double(c.w) * ry;
+        if (kMode == kResidualInitial)
         {
-            const auto c = L.coeff(lv.coeff, x, y);
-            const double rx = r.x, ry = r.y;
-            mine.x += rx / double(c.z) * rx + ry / double(c.w) * ry;
-            if (kMode == kResidualInitial)
-            {
-                const T2 v = static_cast<const T2*>(f)[n];
-                mine.y += double(c.z) * double(v.x) * double(v.x) + double(c.w) * double(v.y) * double(v.y);
-                mine.z += double(c.z) + double(c.w);
-            }
+            const T2 v = static_cast<const T2*>(f)[n];
+            mine.y += double(c.z) * double(v.x) * double(v.x) + double(c.w) * double(v.y) * double(v.y);
+            mine.z += double(c.z) + double(c.w);
+            static_cast<T2*>(lv.x)[n] = T2{r.x * half.x, r.y * half.y};
         }
     }
-    if (kMode == kResidualPlain)
-        return;
     double4 total;
     if (visc_arrive_last<kViscThreads>(partial, counter, blockIdx.x, gridDim.x, block_reduce4<kViscThreads>(mine, 0),
             &total, 0))
@@ -518,183 +505,298 @@ __device__ __forceinline__ double transfer_weight(int fx, int fy, int px, int py
     return result;
 }
 
-// Coarse right-hand side: transpose of the prolongation applied to the fine residual.
-template <typename T>
-__global__ void __launch_bounds__(kViscThreads) k_visc_restrict(ViscLevel fine, ViscLevel coarse, const ViscState* state)
+// Coarse tile of a restriction block, and the fine nodes its stencils cover.
+constexpr int kViscTileX = 32, kViscTileY = 8;
+constexpr int kViscFineX = 2 * kViscTileX + 2, kViscFineY = 2 * kViscTileY + 2;
+
+// The coarse right-hand side at node (px, py): the transpose of the prolongation applied to the 4 x 4
+// fine residuals 2p - 1 .. 2p + 2, q(row, column), summed in the stencil's row order.
+template <typename T, typename Q>
+__device__ __forceinline__ typename Vec<T>::two restrict_node(int px, int py, int cw, int ch, int fw, int fh, Q&& q)
 {
-    allow_dependents();
-    dependency_wait();
-    using T2 = typename Vec<T>::two;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= (coarse.w + 1) * (coarse.h + 1))
-        return;
-    const int px = n % (coarse.w + 1), py = n / (coarse.w + 1);
     double value[2] = {0.0, 0.0};
-    if (!visc_stopped(state))
+    if (px >= 2 && py >= 2 && px <= cw - 3 && py <= ch - 3)
     {
-        // The 4 x 4 fine nodes 2p - 1 .. 2p + 2 cover both components' stencils; they are loaded
-        // together (indices clamped into the lattice, the clamped copies unused), then summed in
-        // the stencil's row order, skipping nodes outside the lattice.
-        const T2* res = static_cast<const T2*>(fine.res);
-        T2 q[4][4];
+        // No clamp reaches a node two or more from every edge: each stencil weight is the
+        // product of the 1D weights (1/2, 1, 1/2) along the face's own axis and
+        // (1/4, 3/4, 3/4, 1/4) across it, exactly transfer_weight's value.
+        constexpr double kNear[3] = {0.5, 1.0, 0.5};
+        constexpr double kFar[4] = {0.25, 0.75, 0.75, 0.25};
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int y = 0; y < 4; ++y)
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-            {
-                const int qx = clampi(2 * px + i - 1, 0, fine.w), qy = clampi(2 * py + j - 1, 0, fine.h);
-                q[j][i] = res[(long long)qy * (fine.w + 1) + qx];
-            }
-        if (px >= 2 && py >= 2 && px <= coarse.w - 3 && py <= coarse.h - 3)
-        {
-            // No clamp reaches a node two or more from every edge: each stencil weight is the
-            // product of the 1D weights (1/2, 1, 1/2) along the face's own axis and
-            // (1/4, 3/4, 3/4, 1/4) across it, exactly transfer_weight's value.
-            constexpr double kNear[3] = {0.5, 1.0, 0.5};
-            constexpr double kFar[4] = {0.25, 0.75, 0.75, 0.25};
+            for (int x = 0; x < 3; ++x)
+                value[0] += kNear[x] * kFar[y] * double(q(y, x).x);
 #pragma unroll
-            for (int y = 0; y < 4; ++y)
+        for (int y = 0; y < 3; ++y)
 #pragma unroll
-                for (int x = 0; x < 3; ++x)
-                    value[0] += kNear[x] * kFar[y] * double(q[y][x].x);
-#pragma unroll
-            for (int y = 0; y < 3; ++y)
-#pragma unroll
-                for (int x = 0; x < 4; ++x)
-                    value[1] += kFar[x] * kNear[y] * double(q[y][x].y);
-        }
-        else
-#pragma unroll
+            for (int x = 0; x < 4; ++x)
+                value[1] += kFar[x] * kNear[y] * double(q(y, x).y);
+    }
+    else
+    {
+#pragma unroll 1
         for (int component = 0; component < 2; ++component)
         {
-            if ((component == 0 && (px == 0 || px == coarse.w || py == coarse.h)) ||
-                (component == 1 && (py == 0 || py == coarse.h || px == coarse.w)))
+            if ((component == 0 && (px == 0 || px == cw || py == ch)) ||
+                (component == 1 && (py == 0 || py == ch || px == cw)))
                 continue;
             const int ex = component == 1 ? 2 : 1, ey = component == 1 ? 1 : 2;
-#pragma unroll
-            for (int y = -1; y <= 2; ++y)
-#pragma unroll
-                for (int x = -1; x <= 2; ++x)
+#pragma unroll 1
+            for (int y = -1; y <= ey; ++y)
+#pragma unroll 1
+                for (int x = -1; x <= ex; ++x)
                 {
                     const int qx = 2 * px + x, qy = 2 * py + y;
-                    if (x > ex || y > ey || qx < 0 || qy < 0 || qx > fine.w || qy > fine.h)
+                    if (qx < 0 || qy < 0 || qx > fw || qy > fh)
                         continue;
-                    const T2 r = q[y + 1][x + 1];
-                    value[component] += transfer_weight(qx, qy, px, py, component, coarse.w, coarse.h) *
+                    const auto r = q(y + 1, x + 1);
+                    value[component] += transfer_weight(qx, qy, px, py, component, cw, ch) *
                                         double(component == 0 ? r.x : r.y);
                 }
         }
     }
-    T2 out;
-    out.x = T(value[0]);
-    out.y = T(value[1]);
-    static_cast<T2*>(coarse.rhs)[n] = out;
+    return {T(value[0]), T(value[1])};
 }
 
-// Fine x += bilinear interpolation of the coarse correction, on valid faces (into fine.next).
+// Residual of the fine level and its restriction in one kernel: a block forms the residuals under
+// its coarse tile in shared memory (66 x 18 of them for 64 x 16 fine nodes of its own, 16 % more work
+// than a pass of its own, against 16 bytes a node written and read back and a launch), then each
+// thread restricts one coarse node, and starts the coarse level's sweep from zero (`start`: the
+// level is smoothed by kernels of its own).
 template <typename T>
-__global__ void __launch_bounds__(kViscThreads) k_visc_prolong(ViscLevel fine, ViscLevel coarse,
-    const unsigned char* solid, const ViscState* state)
-{
-    allow_dependents();
-    dependency_wait();
-    using T2 = typename Vec<T>::two;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= (fine.w + 1) * (fine.h + 1))
-        return;
-    const int px = n % (fine.w + 1), py = n / (fine.w + 1);
-    T2 out;
-    out.x = out.y = T(0);
-    if (!visc_stopped(state))
-    {
-        const T2 own = static_cast<const T2*>(fine.x)[n];
-        const T2* c = static_cast<const T2*>(coarse.x);
-        T value[2] = {own.x, own.y};
-#pragma unroll
-        for (int component = 0; component < 2; ++component)
-        {
-            int bx, by;
-            double tx, ty;
-            transfer_axis(px, component == 1, bx, tx);
-            transfer_axis(py, component == 0, by, ty);
-#pragma unroll
-            for (int y = 0; y < 2; ++y)
-#pragma unroll
-                for (int x = 0; x < 2; ++x)
-                {
-                    int cx, cy;
-                    transfer_clamp(bx + x, by + y, component, coarse.w, coarse.h, cx, cy);
-                    const T2 v = c[(long long)cy * (coarse.w + 1) + cx];
-                    value[component] += T((x == 1 ? tx : 1.0 - tx) * (y == 1 ? ty : 1.0 - ty)) * (component == 0 ? v.x : v.y);
-                }
-        }
-        const FaceMask m = face_mask(fine.w, fine.h, px, py, solid);
-        out.x = m.u ? value[0] : T(0);
-        out.y = m.v ? value[1] : T(0);
-    }
-    static_cast<T2*>(fine.next)[n] = out;
-}
-
-// Coarsest level: 16 damped-Jacobi sweeps from zero in one block's shared memory
-// (ViscosityKernels.h "coarse_smooth").
-template <typename T>
-__global__ void __launch_bounds__(kViscCoarseNodes) k_visc_coarse(ViscLevel lv, double dt, const unsigned char* solid,
-    const ViscState* state)
+__global__ void __launch_bounds__(kViscThreads) k_visc_restrict(ViscLevel fine, ViscLevel coarse, double dt, const void* b,
+    int start, const ViscState* state)
 {
     allow_dependents();
     dependency_wait();
     using T2 = typename Vec<T>::two;
     using T4 = typename Vec<T>::four;
-    __shared__ T2 sx[kViscCoarseNodes];
-    __shared__ T4 sc[kViscCoarseNodes];
-    const int nodes = (lv.w + 1) * (lv.h + 1);
-    const int n = threadIdx.x;
-    const bool mine = n < nodes;
-    const bool stopped = visc_stopped(state);
-    const int x = mine ? n % (lv.w + 1) : 0, y = mine ? n / (lv.w + 1) : 0;
-    T2 b;
-    b.x = b.y = T(0);
-    if (mine)
+    __shared__ T2 res[kViscFineY][kViscFineX];
+    if (visc_stopped(state))
+        return;
+    const int X0 = blockIdx.x * kViscTileX, Y0 = blockIdx.y * kViscTileY;
+    for (int i = threadIdx.x; i < kViscFineX * kViscFineY; i += kViscThreads)
     {
-        sx[n] = T2{T(0), T(0)};
-        sc[n] = static_cast<const T4*>(lv.coeff)[n];
-        b = static_cast<const T2*>(lv.rhs)[n];
+        const int j = i / kViscFineX, k = i - j * kViscFineX;
+        const int x = 2 * X0 - 1 + k, y = 2 * Y0 - 1 + j;
+        T2 r{T(0), T(0)};
+        if (x >= 0 && y >= 0 && x <= fine.w && y <= fine.h)
+        {
+            const Around o = around(fine.w, fine.h, x, y);
+            T ax, ay;
+            operator_at<T>(static_cast<const T2*>(fine.x), o, static_cast<const T4*>(fine.coeff), o, T(dt), ax, ay);
+            const T2 bb = static_cast<const T2*>(b)[o.own], half = static_cast<const T2*>(fine.half)[o.own];
+            r.x = half.x != T(0) ? bb.x - ax : T(0);
+            r.y = half.y != T(0) ? bb.y - ay : T(0);
+        }
+        res[j][k] = r;
     }
     __syncthreads();
-    // Shared-memory views of the level with the clamped accessors of Nodes.
-    auto at = [&](int px, int py) { return clampi(py, 0, lv.h) * (lv.w + 1) + clampi(px, 0, lv.w); };
-    const FaceMask m = face_mask(lv.w, lv.h, x, y, solid);
-    for (int sweep = 0; sweep < 16 && !stopped; ++sweep)
+    const int lx = threadIdx.x % kViscTileX, ly = threadIdx.x / kViscTileX;
+    const int px = X0 + lx, py = Y0 + ly;
+    if (px > coarse.w || py > coarse.h)
+        return;
+    const T2 out = restrict_node<T>(px, py, coarse.w, coarse.h, fine.w, fine.h,
+        [&](int j, int i) { return res[2 * ly + j][2 * lx + i]; });
+    const int n = py * (coarse.w + 1) + px;
+    static_cast<T2*>(coarse.rhs)[n] = out;
+    if (start)
     {
-        T2 value;
-        value.x = value.y = T(0);
-        if (mine)
-        {
-            const T dtt = T(dt);
-            auto shear = [&](int px, int py)
+        const T2 half = static_cast<const T2*>(coarse.half)[n];
+        static_cast<T2*>(coarse.x)[n] = T2{out.x * half.x, out.y * half.y};
+    }
+}
+
+// x plus the bilinear interpolation of the coarse correction at fine node (px, py), on valid faces;
+// `coarse` is the correction's lattice, cw x ch cells.
+template <typename T>
+__device__ __forceinline__ typename Vec<T>::two prolong_node(const typename Vec<T>::two& own,
+    const typename Vec<T>::two& half, const typename Vec<T>::two* coarse, int cw, int ch, int px, int py)
+{
+    T value[2] = {own.x, own.y};
+#pragma unroll
+    for (int component = 0; component < 2; ++component)
+    {
+        int bx, by;
+        double tx, ty;
+        transfer_axis(px, component == 1, bx, tx);
+        transfer_axis(py, component == 0, by, ty);
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
             {
-                const T2 p = sx[at(px, py)];
-                return sc[at(px, py)].y * ((p.x - sx[at(px, py - 1)].x) + (p.y - sx[at(px - 1, py)].y));
-            };
-            const T2 c = sx[at(x, y)];
-            const T4 a = sc[at(x, y)];
-            const T t = shear(x, y);
-            const T nx = T(2) * (sc[at(x - 1, y)].x * (c.x - sx[at(x - 1, y)].x) + a.x * (c.x - sx[at(x + 1, y)].x));
-            const T ny = T(2) * (sc[at(x, y - 1)].x * (c.y - sx[at(x, y - 1)].y) + a.x * (c.y - sx[at(x, y + 1)].y));
-            const T ax = a.z * c.x + dtt * (nx + (t - shear(x, y + 1)));
-            const T ay = a.w * c.y + dtt * (ny + (t - shear(x + 1, y)));
-            const T dxx = a.z + dtt * (T(2) * (a.x + sc[at(x - 1, y)].x) + a.y + sc[at(x, y + 1)].y);
-            const T dyy = a.w + dtt * (T(2) * (a.x + sc[at(x, y - 1)].x) + a.y + sc[at(x + 1, y)].y);
-            value.x = m.u ? c.x + T(0.5) * (b.x - ax) / dxx : T(0);
-            value.y = m.v ? c.y + T(0.5) * (b.y - ay) / dyy : T(0);
+                int cx, cy;
+                transfer_clamp(bx + x, by + y, component, cw, ch, cx, cy);
+                const auto v = coarse[cy * (cw + 1) + cx];
+                value[component] += T((x == 1 ? tx : 1.0 - tx) * (y == 1 ? ty : 1.0 - ty)) * (component == 0 ? v.x : v.y);
+            }
+    }
+    return {half.x != T(0) ? value[0] : T(0), half.y != T(0) ? value[1] : T(0)};
+}
+
+// The prolongation and the first post-smoothing sweep in one kernel: a block forms the prolonged
+// solution of its 32 x 8 nodes and the ring around them in shared memory (1.33 times the nodes,
+// against 16 bytes a node written and read back and a launch), then sweeps them (into fine.next).
+template <typename T>
+__global__ void __launch_bounds__(kViscThreads) k_visc_prolong_smooth(ViscLevel fine, ViscLevel coarse, double dt,
+    const void* b, const ViscState* state)
+{
+    allow_dependents();
+    dependency_wait();
+    using T2 = typename Vec<T>::two;
+    using T4 = typename Vec<T>::four;
+    constexpr int RX = kViscTileX + 2, RY = kViscTileY + 2;
+    __shared__ T2 tile[RY * RX];
+    if (visc_stopped(state))
+        return;
+    const int X0 = blockIdx.x * kViscTileX, Y0 = blockIdx.y * kViscTileY;
+    for (int i = threadIdx.x; i < RX * RY; i += kViscThreads)
+    {
+        // Clamped like the operator's reads: the ring beyond the lattice repeats its edge.
+        const int j = i / RX, k = i - j * RX;
+        const int x = clampi(X0 - 1 + k, 0, fine.w), y = clampi(Y0 - 1 + j, 0, fine.h);
+        const int n = y * (fine.w + 1) + x;
+        tile[i] = prolong_node<T>(static_cast<const T2*>(fine.x)[n], static_cast<const T2*>(fine.half)[n],
+            static_cast<const T2*>(coarse.x), coarse.w, coarse.h, x, y);
+    }
+    __syncthreads();
+    const int lx = threadIdx.x % kViscTileX, ly = threadIdx.x / kViscTileX;
+    const int x = X0 + lx, y = Y0 + ly;
+    if (x > fine.w || y > fine.h)
+        return;
+    const int at = (ly + 1) * RX + lx + 1;
+    const Around t{at, at - 1, at + 1, at - RX, at + RX, at + RX - 1, at - RX + 1};
+    const Around o = around(fine.w, fine.h, x, y);
+    T ax, ay;
+    operator_at<T>(tile, t, static_cast<const T4*>(fine.coeff), o, T(dt), ax, ay);
+    static_cast<T2*>(fine.next)[o.own] =
+        jacobi<T>(tile[at], static_cast<const T2*>(b)[o.own], static_cast<const T2*>(fine.half)[o.own], ax, ay);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Coarse tail: the small levels cycled by one CTA in shared memory
+// ---------------------------------------------------------------------------------------------
+
+// Below a few thousand nodes a pass is nothing but its launch (2.5 to 3 us each, five passes a level),
+// so the V-cycle's last levels run in one CTA: coefficients, half inverse diagonals, right-hand sides
+// and two solutions of every level in shared memory, a barrier between passes. The coarsest level
+// takes 16 damped-Jacobi sweeps from zero (ViscosityKernels.h "coarse_smooth").
+constexpr int kViscTailThreads = 1024;
+constexpr int kViscTailLevels = 8;
+
+struct ViscTail
+{
+    int levels;
+    ViscLevel lev[kViscTailLevels];
+};
+
+// Shared-memory bytes of one node of a tail level: four coefficients, two half inverse diagonals, the
+// right-hand side and two solutions.
+__host__ __device__ inline size_t visc_tail_bytes(int nodes, size_t elem) { return size_t(nodes) * 12 * elem; }
+
+constexpr size_t kViscTailMaxBytes = 200 * 1024;
+extern __shared__ __align__(16) unsigned char visc_smem[];
+
+template <typename T>
+__global__ void __launch_bounds__(kViscTailThreads) k_visc_tail(const ViscTail tail, double dt, const ViscState* state)
+{
+    allow_dependents();
+    using T2 = typename Vec<T>::two;
+    using T4 = typename Vec<T>::four;
+    const T step = T(dt);
+    // Level l's arrays: node counts add up, each array of all levels together.
+    int base[kViscTailLevels + 1];
+    base[0] = 0;
+#pragma unroll
+    for (int l = 0; l < kViscTailLevels; ++l)
+        base[l + 1] = base[l] + (l < tail.levels ? (tail.lev[l].w + 1) * (tail.lev[l].h + 1) : 0);
+    const int total = base[kViscTailLevels];
+    T4* const coeff = reinterpret_cast<T4*>(visc_smem);
+    T2* const half = reinterpret_cast<T2*>(coeff + total);
+    T2* const rhs = half + total;
+    T2* const xs = rhs + total;
+    T2* const ys = xs + total;
+    // Written once per solve, long before this launch: read ahead of the wait.
+#pragma unroll
+    for (int l = 0; l < kViscTailLevels; ++l)
+        if (l < tail.levels)
+            for (int n = threadIdx.x; n < base[l + 1] - base[l]; n += kViscTailThreads)
+            {
+                coeff[base[l] + n] = static_cast<const T4*>(tail.lev[l].coeff)[n];
+                half[base[l] + n] = static_cast<const T2*>(tail.lev[l].half)[n];
+            }
+    dependency_wait();
+    if (visc_stopped(state))
+        return;
+    for (int n = threadIdx.x; n < base[1]; n += kViscTailThreads)
+        rhs[n] = static_cast<const T2*>(tail.lev[0].rhs)[n];
+    __syncthreads();
+    // One Jacobi sweep of level l (first node at o) from x to y.
+    auto sweep = [&](int w, int h, int o, const T2* x, T2* y)
+    {
+        for (int n = threadIdx.x; n < (w + 1) * (h + 1); n += kViscTailThreads)
+        {
+            const Around a = around(w, h, n % (w + 1), n / (w + 1));
+            T ax, ay;
+            operator_at<T>(x + o, a, coeff + o, a, step, ax, ay);
+            y[o + n] = jacobi<T>(x[o + n], rhs[o + n], half[o + n], ax, ay);
         }
         __syncthreads();
-        if (mine)
-            sx[n] = value;
+    };
+#pragma unroll 1
+    for (int l = 0; l < tail.levels; ++l)
+    {
+        const int w = tail.lev[l].w, h = tail.lev[l].h, o = base[l], nodes = (w + 1) * (h + 1);
+        for (int n = threadIdx.x; n < nodes; n += kViscTailThreads)
+            xs[o + n] = T2{rhs[o + n].x * half[o + n].x, rhs[o + n].y * half[o + n].y};
+        __syncthreads();
+        if (l + 1 == tail.levels)
+        {
+            // The first of the 16 sweeps is the one from zero.
+#pragma unroll 1
+            for (int i = 1; i < 16; i += 2)
+            {
+                sweep(w, h, o, xs, ys);
+                if (i + 1 < 16)
+                    sweep(w, h, o, ys, xs);
+            }
+            break;
+        }
+        sweep(w, h, o, xs, ys);
+        // The residual of ys goes to xs, which the up leg's prolongation overwrites.
+        for (int n = threadIdx.x; n < nodes; n += kViscTailThreads)
+        {
+            const Around a = around(w, h, n % (w + 1), n / (w + 1));
+            T ax, ay;
+            operator_at<T>(ys + o, a, coeff + o, a, step, ax, ay);
+            xs[o + n] = T2{half[o + n].x != T(0) ? rhs[o + n].x - ax : T(0), half[o + n].y != T(0) ? rhs[o + n].y - ay : T(0)};
+        }
+        __syncthreads();
+        const int cw = tail.lev[l + 1].w, ch = tail.lev[l + 1].h, co = base[l + 1];
+        for (int n = threadIdx.x; n < (cw + 1) * (ch + 1); n += kViscTailThreads)
+        {
+            const int px = n % (cw + 1), py = n / (cw + 1);
+            rhs[co + n] = restrict_node<T>(px, py, cw, ch, w, h,
+                [&](int j, int i) { return xs[o + clampi(2 * py + j - 1, 0, h) * (w + 1) + clampi(2 * px + i - 1, 0, w)]; });
+        }
         __syncthreads();
     }
-    if (mine)
-        static_cast<T2*>(lv.x)[n] = stopped ? T2{T(0), T(0)} : sx[n];
+    // Up: the solution of level l is in ys.
+#pragma unroll 1
+    for (int l = tail.levels - 2; l >= 0; --l)
+    {
+        const int w = tail.lev[l].w, h = tail.lev[l].h, o = base[l];
+        const int cw = tail.lev[l + 1].w, ch = tail.lev[l + 1].h, co = base[l + 1];
+        for (int n = threadIdx.x; n < (w + 1) * (h + 1); n += kViscTailThreads)
+            ys[o + n] = prolong_node<T>(ys[o + n], half[o + n], ys + co, cw, ch, n % (w + 1), n / (w + 1));
+        __syncthreads();
+        sweep(w, h, o, ys, xs);
+        sweep(w, h, o, xs, ys);
+    }
+    for (int n = threadIdx.x; n < base[1]; n += kViscTailThreads)
+        static_cast<T2*>(tail.lev[0].x)[n] = ys[n];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -733,7 +835,9 @@ __global__ void __launch_bounds__(kViscThreads) k_visc_dot_rz(int nodes, const v
             if (n < nodes)
             {
                 mine.x += double(a[k].x) * double(b[k].x) + double(a[k].y) * double(b[k].y);
-                mine.y += double(a[k].x) / double(c[k].z) * double(a[k].x) + double(a[k].y) / double(c[k].w) * double(a[k].y);
+                // r.x^2 / m.u + r.y^2 / m.v over one division.
+                const double mu = double(c[k].z), mv = double(c[k].w), rx = double(a[k].x), ry = double(a[k].y);
+                mine.y += (rx * rx * mv + ry * ry * mu) / (mu * mv);
             }
         }
     }
@@ -781,10 +885,10 @@ __global__ void __launch_bounds__(kViscThreads) k_visc_direction(int nodes, cons
     static_cast<T2*>(d)[n] = out;
 }
 
-// x += alpha d, r -= alpha q.
+// x += alpha d, r -= alpha q, and the next V-cycle's sweep from zero, r / (2 D), into `start`.
 template <typename T>
 __global__ void __launch_bounds__(kViscThreads) k_visc_update(int nodes, void* x, void* r, const void* d, const void* q,
-    const ViscState* state)
+    const void* half, void* start, const ViscState* state)
 {
     allow_dependents();
     dependency_wait();
@@ -801,6 +905,8 @@ __global__ void __launch_bounds__(kViscThreads) k_visc_update(int nodes, void* x
     b.y -= alpha * qq.y;
     static_cast<T2*>(x)[n] = a;
     static_cast<T2*>(r)[n] = b;
+    const T2 hd = static_cast<const T2*>(half)[n];
+    static_cast<T2*>(start)[n] = T2{b.x * hd.x, b.y * hd.y};
 }
 
 // solution = face velocities on valid faces, rhs = mass * solution.
@@ -841,14 +947,19 @@ __global__ void __launch_bounds__(kViscThreads) k_visc_unpack(int w, int h, cons
 
 // Restart from the true residual after the recurrence claimed convergence too early.
 template <typename T>
-__global__ void __launch_bounds__(kViscThreads) k_visc_refresh(int nodes, const void* truth, void* r, ViscState* state)
+__global__ void __launch_bounds__(kViscThreads) k_visc_refresh(int nodes, const void* truth, void* r, const void* half,
+    void* start, ViscState* state)
 {
     allow_dependents();
     dependency_wait();
     using T2 = typename Vec<T>::two;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n < nodes)
-        static_cast<T2*>(r)[n] = static_cast<const T2*>(truth)[n];
+    {
+        const T2 b = static_cast<const T2*>(truth)[n], hd = static_cast<const T2*>(half)[n];
+        static_cast<T2*>(r)[n] = b;
+        static_cast<T2*>(start)[n] = T2{b.x * hd.x, b.y * hd.y};
+    }
     if (n == 0)
     {
         state->rz = state->alpha = state->beta = 0.0;
