@@ -384,38 +384,43 @@ __global__ void __launch_bounds__(32 * WARPS, (sizeof(T) == 4 && WARPS == 8) ? 2
             strip_sweep<T, K, WARPS>(s, edges, 0, false, 0, lane, warp);
             strip_sweep<T, K, WARPS>(s, edges, 1, false, 1, lane, warp);
         }
-        // Residual of every cell, summed along x into the lines; the edge buffers hold the final
-        // values: buffer 0 colour 0, buffer 1 colour 1.
-        const T above_a = edges.bottom[1][warp][lane], above_b = edges.bottom[0][warp][lane];
-        const T below_a = edges.top[0][warp + 2][lane], below_b = edges.top[1][warp + 2][lane];
+        // Residual, summed along x into the lines. The last half-sweep solved the equations of its
+        // colour (1), so only cells of colour 0 have a residual (column 2j in even rows, 2j + 1 in
+        // odd ones): half the terms and shuffles of a residual of every cell (whole projections:
+        // 2048 x 2048 16.41 -> 16.15 ms, 1920 x 1080 in mixed precision 11.61 -> 11.22 ms). Edge
+        // buffer 1 holds colour 1's final values.
+        const T above_a = edges.bottom[1][warp][lane], below_b = edges.top[1][warp + 2][lane];
         const int gx = X0 + 2 * lane;
 #pragma unroll
         for (int k = 0; k < K; ++k)
         {
-            T left = __shfl_up_sync(0xffffffffu, s.b[k], 1);
-            T right = __shfl_down_sync(0xffffffffu, s.a[k], 1);
-            left = lane == 0 ? T(0) : left;
-            right = lane == 31 ? T(0) : right;
-            const T ua = k == 0 ? above_a : s.a[k - 1];
-            const T ub = k == 0 ? above_b : s.b[k - 1];
-            const T na_ = k == K - 1 ? below_a : s.a[k + 1];
-            const T nb_ = k == K - 1 ? below_b : s.b[k + 1];
-            const T wua = k == 0 ? s.ua : s.da[k - 1];
-            const T wub = k == 0 ? s.ub : s.db[k - 1];
             const T a = s.a[k], b = s.b[k];
-            // Lane 0's cells are halo columns whose residual neither the output nor the
-            // restriction reads (its first lane, HALO/2, takes columns from HALO - 1 on).
-            T wl = __shfl_up_sync(0xffffffffu, s.wr[k], 1); // every lane takes part
-            wl = lane == 0 ? T(0) : wl;
-            const T pa = (wl * (a - left) + s.wm[k] * (a - b)) + (wua * (a - ua) + s.da[k] * (a - na_));
-            const T pb = (s.wm[k] * (b - a) + s.wr[k] * (b - right)) + (wub * (b - ub) + s.db[k] * (b - nb_));
             const int y = warp * K + k;
-            const T res_a = s.ia[k] > T(0) ? s.ra[k] - pa : T(0);
-            const T res_b = s.ib[k] > T(0) ? s.rb[k] - pb : T(0);
-            // Lanes 0 and 31 hold no coarse column, so the wrapped shuffles are never summed.
-            const T res_left = __shfl_up_sync(0xffffffffu, res_b, 1);
-            const T res_right = __shfl_down_sync(0xffffffffu, res_a, 1);
-            lines[y][lane] = restrict_sum(along_x, res_left, res_a, res_b, res_right);
+            // Lanes 0 and 31 hold no coarse column, and lane 0's cells are halo columns whose residual
+            // neither the output nor the restriction reads (its first lane, HALO/2, takes columns
+            // from HALO - 1 on), so the wrapped shuffles are never summed.
+            T sum;
+            if (k % 2 == 0)
+            {
+                const T left = __shfl_up_sync(0xffffffffu, b, 1);
+                const T wl = __shfl_up_sync(0xffffffffu, s.wr[k], 1);
+                const T up = k == 0 ? above_a : s.a[k - 1];
+                const T wu = k == 0 ? s.ua : s.da[k - 1];
+                const T pa = (wl * (a - left) + s.wm[k] * (a - b)) + (wu * (a - up) + s.da[k] * (a - s.a[k + 1]));
+                const T res = s.ia[k] > T(0) ? s.ra[k] - pa : T(0);
+                const T res_right = __shfl_down_sync(0xffffffffu, res, 1);
+                sum = along_x.w[1] * res + along_x.w[3] * res_right;
+            }
+            else
+            {
+                const T right = __shfl_down_sync(0xffffffffu, a, 1);
+                const T dn = k == K - 1 ? below_b : s.b[k + 1];
+                const T pb = (s.wm[k] * (b - a) + s.wr[k] * (b - right)) + (s.db[k - 1] * (b - s.b[k - 1]) + s.db[k] * (b - dn));
+                const T res = s.ib[k] > T(0) ? s.rb[k] - pb : T(0);
+                const T res_left = __shfl_up_sync(0xffffffffu, res, 1);
+                sum = along_x.w[0] * res_left + along_x.w[2] * res;
+            }
+            lines[y][lane] = sum;
             const int gy = Y0 + y;
             if (y >= Shape::HALO && y < Shape::HALO + Shape::OY && 2 * lane >= Shape::HALO &&
                 2 * lane < Shape::HALO + Shape::OX && gy < Lh && gx < Lw)
