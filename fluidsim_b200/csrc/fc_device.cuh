@@ -145,7 +145,7 @@ struct GridDesc
     // face velocities, unpadded: u is (W+1) x H, v is W x (H+1), row-major
     void* u;
     void* v;
-    // coarsest inverse, row-major FP64 (k_coarse_inverse), and the tail's layout and transfer tables
+    // coarsest inverse, row-major FP64 (k_rebuild_tail), and the tail's layout and transfer tables
     // (TailTable, fc_tail.cuh)
     double* coarse_inverse;
     const void* tail_table;

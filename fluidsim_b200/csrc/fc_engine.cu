@@ -1029,7 +1029,7 @@ struct Plan
     std::vector<int> post0_shape; // per grid
     int max_levels = 0;
     int max_tail = 0;
-    int padded_max[kMaxLevels] = {}; // largest padded level array of any grid, per level
+    int cells_max[kMaxLevels] = {}; // most cells of any grid's level, per level
     size_t tail_smem = 0;
     int tail_threads = 0;
     cudaGraphExec_t exec = nullptr;
@@ -1146,7 +1146,7 @@ std::unique_ptr<Plan> make_plan(const std::vector<Grid*>& grids, cudaStream_t st
         plan->tail_smem = std::max(plan->tail_smem, g->tail_smem);
         plan->tail_threads = std::max(plan->tail_threads, g->tail_threads);
         for (size_t l = 0; l < g->levels.size(); ++l)
-            plan->padded_max[l] = std::max(plan->padded_max[l], g->levels[l].S * (g->levels[l].h + 2));
+            plan->cells_max[l] = std::max(plan->cells_max[l], g->levels[l].w * g->levels[l].h);
     }
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, grids.front()->device);
@@ -1217,24 +1217,18 @@ std::unique_ptr<Plan> make_plan(const std::vector<Grid*>& grids, cudaStream_t st
 // Launch sequences
 // ------------------------------------------------------------------------------------------
 
-// Density, face weights, multigrid conductances and the coarsest inverse of every grid.
+// Face weights, multigrid conductances and the coarsest inverse of every grid.
 // The kernels are launched with programmatic serialization: each starts with dependent_start(),
 // so its launch overlaps the end of its predecessor.
 template <typename T> void launch_rebuild(Plan& p)
 {
     cudaStream_t s = p.stream;
-    FC_LAUNCH_DEP(k_density, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec));
     FC_LAUNCH_DEP(k_coefficients<T>, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec));
-    for (int l = 0; l + 1 < p.max_levels; ++l)
-        FC_LAUNCH_DEP(k_coarsen<T>, dim3(ceil_div(p.padded_max[l + 1], 256), p.n()), 256, 0, s, p.d_desc, l);
-    if (p.precision == FC_PRECISION_MIXED)
-        for (int l = 1; l < p.max_tail; ++l)
-            FC_LAUNCH_DEP(k_weights_half, dim3(ceil_div(p.padded_max[l], 256), p.n()), 256, 0, s, p.d_desc, l);
-    // Level by level: under Dirichlet air a coarse level's held cells follow from the finer
-    // level's inverse diagonal, and the coarsest factor from the level above it.
-    for (int l = 0; l + 1 < p.max_levels; ++l)
-        FC_LAUNCH_DEP(k_inverse_diagonal<T>, dim3(ceil_div(p.padded_max[l], 256), p.n()), 256, 0, s, p.d_desc, l);
-    FC_LAUNCH_DEP(k_coarse_inverse<T>, p.n(), kCoarseThreads, 0, s, p.d_desc);
+    // Level by level: a coarse level follows from the finer one's weights and, under Dirichlet air,
+    // its held cells from the finer level's inverse diagonal.
+    for (int l = 0; l < p.max_tail; ++l)
+        FC_LAUNCH_DEP(k_rebuild_level<T>, dim3(ceil_div(p.cells_max[l + 1], 256), p.n()), 256, 0, s, p.d_desc, l);
+    FC_LAUNCH_DEP(k_rebuild_tail<T>, p.n(), kCoarseThreads, 0, s, p.d_desc);
 }
 
 // Resident CTAs of the persistent smoothing kernels: two per SM in FP32, one in FP64 (their

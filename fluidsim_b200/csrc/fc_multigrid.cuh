@@ -12,8 +12,8 @@
 //    fine-level z reductions fused into the post kernel.
 //  * k_mg_tail (fc_tail.cuh): the coarse levels of at most 64 x 64 cells are cycled by one CTA per
 //    grid as register strips, including the coarsest direct solve (an explicit FP64 inverse).
-//  * The rebuild: k_coarsen (one coarse cell per thread), k_inverse_diagonal, k_weights_half
-//    (mixed precision) and k_coarse_inverse (fc_tail.cuh).
+//  * The rebuild: k_rebuild_level (one coarse cell per thread) down to the tail, then
+//    k_rebuild_tail (fc_tail.cuh) for the rest and the coarsest inverse.
 #pragma once
 
 #include "fc_device.cuh"
@@ -86,28 +86,6 @@ __global__ void __launch_bounds__(kVecThreads) k_precondition_diagonal(const Gri
 // Rebuild: coarse conductances and the coarsest inverse
 // ------------------------------------------------------------------------------------------
 
-// Mixed precision: FP16 copies of a level's face weights for the strip kernels, divided by
-// the level's scale and saturated at the largest finite FP16 value (blockIdx.y = grid).
-__global__ void k_weights_half(const GridDesc* __restrict__ grids, int level)
-{
-    dependent_start();
-    const GridDesc& g = grids[blockIdx.y];
-    if (level < 1 || level >= g.tail)
-        return;
-    const LevelDesc& L = g.lev[level];
-    const int n = L.S * (L.h + 2);
-    const float inv = 1.0f / L.wscale;
-    const float* right = static_cast<const float*>(L.right);
-    const float* down = static_cast<const float*>(L.down);
-    __half* rh = static_cast<__half*>(const_cast<void*>(L.right_h));
-    __half* dh = static_cast<__half*>(const_cast<void*>(L.down_h));
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    {
-        rh[i] = __float2half_rn(fminf(right[i] * inv, 65504.0f));
-        dh[i] = __float2half_rn(fminf(down[i] * inv, 65504.0f));
-    }
-}
-
 // Dirichlet air (no reference counterpart): a cell held at zero. On the fine level the air
 // cells; on a coarse level the cells none of whose fine cells (2x .. 2x+1, 2y .. 2y+1 of the
 // level above, whose inverse diagonal is final) is an unknown. A held cell keeps its face
@@ -128,87 +106,71 @@ template <typename T> __device__ __forceinline__ bool held_cell(const GridDesc& 
     return true;
 }
 
-// Inverse diagonal of a level the strip kernels smooth (blockIdx.y = grid): for each cell
-// 1 / (((left + right) + up) + down) over its face weights, decoded as the kernels decode them
-// (the FP16 copies times the level scale on mixed-precision coarse levels), 0 where the sum is
-// not positive and in the padding. The kernels formed it per region before; the sum and the
-// reciprocal are the same, so the smoothing is unchanged (PressureMultigrid.cpp:104-117).
-template <typename T> __global__ void k_inverse_diagonal(const GridDesc* __restrict__ grids, int level)
+// FP16 copy of a face weight of a mixed-precision coarse level, divided by the level's scale and
+// saturated at the largest finite FP16 value; the smoothing kernels read it times the scale.
+__device__ __forceinline__ __half half_weight(float w, float inv_scale) { return __float2half_rn(fminf(w * inv_scale, 65504.0f)); }
+
+// Inverse diagonal of cell (x, y) of a smoothed level: 1 / (((left + right) + up) + down) over its
+// face weights as the kernels decode them (`half`: the FP16 copies times the level scale), 0 where the
+// sum is not positive (PressureMultigrid.cpp:104-117).
+template <typename T>
+__device__ __forceinline__ T inverse_diagonal(const GridDesc& g, const LevelDesc& L, int level, bool half, int x, int y)
 {
-    dependent_start();
-    const GridDesc& g = grids[blockIdx.y];
-    if (level + 1 >= g.levels)
-        return;
-    const LevelDesc& L = g.lev[level];
-    const int n = L.S * (L.h + 2);
-    T* inv = static_cast<T*>(L.inv);
+    const long long i = padded_index(L.S, x, y);
+    const T* right = static_cast<const T*>(L.right);
+    const T* down = static_cast<const T*>(L.down);
+    T wl = right[i - 1], wr = right[i], wu = down[i - L.S], wd = down[i];
+    if constexpr (sizeof(T) == 4)
+    {
+        if (half)
+        {
+            const float inv = 1.0f / L.wscale;
+            wl = __half2float(half_weight(wl, inv)) * L.wscale;
+            wr = __half2float(half_weight(wr, inv)) * L.wscale;
+            wu = __half2float(half_weight(wu, inv)) * L.wscale;
+            wd = __half2float(half_weight(wd, inv)) * L.wscale;
+        }
+    }
+    const T diag = ((wl + wr) + wu) + wd;
+    if (g.air && held_cell<T>(g, level, x, y))
+        return T(0);
+    return diag > T(0) ? reciprocal(diag) : T(0);
+}
+
+// Everything that follows from level `level` around coarse cell (x, y) of the next one: the inverse
+// diagonals of its up to four fine cells (and, in mixed precision, the FP16 copies of their weights),
+// and the coarse cell's conductances (PressureMultigrid.cpp:142-202, coarsen).
+template <typename T> __device__ __forceinline__ void rebuild_cell(const GridDesc& g, int level, int x, int y)
+{
+    const LevelDesc& f = g.lev[level];
+    const LevelDesc& c = g.lev[level + 1];
+    const T* fr = static_cast<const T*>(f.right);
+    const T* fd = static_cast<const T*>(f.down);
     bool half = false;
     if constexpr (sizeof(T) == 4)
-        half = L.right_h != nullptr && level >= 1 && level < g.tail;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    {
-        const int x = i % L.S - kPadX, y = i / L.S - 1;
-        T value = T(0);
-        if (x >= 0 && x < L.w && y >= 0 && y < L.h)
+        half = f.right_h != nullptr && level >= 1 && level < g.tail;
+    const int fy_end = min(2 * y + 2, f.h), fx_end = min(2 * x + 2, f.w);
+    for (int fy = 2 * y; fy < fy_end; ++fy)
+        for (int fx = 2 * x; fx < fx_end; ++fx)
         {
-            T wl, wr, wu, wd;
+            const long long i = padded_index(f.S, fx, fy);
+            static_cast<T*>(f.inv)[i] = inverse_diagonal<T>(g, f, level, half, fx, fy);
             if constexpr (sizeof(T) == 4)
             {
                 if (half)
                 {
-                    const __half* rh = static_cast<const __half*>(L.right_h);
-                    const __half* dh = static_cast<const __half*>(L.down_h);
-                    wl = __half2float(rh[i - 1]) * L.wscale;
-                    wr = __half2float(rh[i]) * L.wscale;
-                    wu = __half2float(dh[i - L.S]) * L.wscale;
-                    wd = __half2float(dh[i]) * L.wscale;
+                    const float inv = 1.0f / f.wscale;
+                    static_cast<__half*>(const_cast<void*>(f.right_h))[i] = half_weight(fr[i], inv);
+                    static_cast<__half*>(const_cast<void*>(f.down_h))[i] = half_weight(fd[i], inv);
                 }
             }
-            if (!half)
-            {
-                const T* right = static_cast<const T*>(L.right);
-                const T* down = static_cast<const T*>(L.down);
-                wl = right[i - 1];
-                wr = right[i];
-                wu = down[i - L.S];
-                wd = down[i];
-            }
-            const T diag = ((wl + wr) + wu) + wd;
-            value = diag > T(0) ? reciprocal(diag) : T(0);
-            if (g.air && held_cell<T>(g, level, x, y))
-                value = T(0);
         }
-        inv[i] = value;
-    }
-}
-
-// Coarse level `level + 1` from `level`. PressureMultigrid.cpp:142-202 (coarsen) and
-// :104-117 (the diagonal is recomputed on the fly wherever it is needed).
-// One thread per coarse cell (blockIdx.y = grid): the FP64 divisions of a cell form a long
-// dependent chain, so the kernel needs many cells in flight rather than many cells per thread.
-template <typename T> __global__ void k_coarsen(const GridDesc* __restrict__ grids, int level)
-{
-    dependent_start();
-    const GridDesc& g = grids[blockIdx.y];
-    if (level + 1 >= g.levels)
-        return;
-    const LevelDesc& f = g.lev[level];
-    const LevelDesc& c = g.lev[level + 1];
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= c.w * c.h)
-        return;
-    const int x = q % c.w, y = q / c.w;
-    const T* fr = static_cast<const T*>(f.right);
-    const T* fd = static_cast<const T*>(f.down);
-    T* cr = static_cast<T*>(c.right);
-    T* cd = static_cast<T*>(c.down);
     double right = 0.0, down = 0.0;
     if (x + 1 < c.w)
     {
         const int e = 2 * x + 2;
         const double a = (f.cx[e - 1] - c.cx[x]) / (f.cx[e - 1] - f.cx[e - 2]);
         const double b = e + 1 < f.w ? (c.cx[x + 1] - f.cx[e]) / (f.cx[e + 1] - f.cx[e]) : 0.0;
-        const int fy_end = min(2 * y + 2, f.h);
         for (int fy = 2 * y; fy < fy_end; ++fy)
         {
             const long long i = padded_index(f.S, e - 1, fy); // fine cell 2x+1: its right face is the coarse face
@@ -223,7 +185,6 @@ template <typename T> __global__ void k_coarsen(const GridDesc* __restrict__ gri
         const int e = 2 * y + 2;
         const double a = (f.cy[e - 1] - c.cy[y]) / (f.cy[e - 1] - f.cy[e - 2]);
         const double b = e + 1 < f.h ? (c.cy[y + 1] - f.cy[e]) / (f.cy[e + 1] - f.cy[e]) : 0.0;
-        const int fx_end = min(2 * x + 2, f.w);
         for (int fx = 2 * x; fx < fx_end; ++fx)
         {
             const long long i = padded_index(f.S, fx, e - 1); // fine cell 2y+1: its lower face is the coarse face
@@ -234,8 +195,23 @@ template <typename T> __global__ void k_coarsen(const GridDesc* __restrict__ gri
         }
     }
     const long long ci = padded_index(c.S, x, y);
-    cr[ci] = T(right);
-    cd[ci] = T(down);
+    static_cast<T*>(c.right)[ci] = T(right);
+    static_cast<T*>(c.down)[ci] = T(down);
+}
+
+// The rebuild of one level above the tail (blockIdx.y = grid), one thread per coarse cell: the FP64
+// divisions of a cell form a long dependent chain, so the kernel needs many cells in flight rather
+// than many cells per thread. The levels from the tail on are rebuilt by one CTA (k_rebuild_tail).
+template <typename T> __global__ void k_rebuild_level(const GridDesc* __restrict__ grids, int level)
+{
+    dependent_start();
+    const GridDesc& g = grids[blockIdx.y];
+    if (level >= g.tail)
+        return;
+    const LevelDesc& c = g.lev[level + 1];
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < c.w * c.h)
+        rebuild_cell<T>(g, level, q % c.w, q / c.w);
 }
 
 } // namespace fc

@@ -103,45 +103,24 @@ __device__ __forceinline__ bool held_at(const unsigned char* __restrict__ solid,
     const GridDesc& g = grids[t.grid];                                                             \
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
 
-// Density from component masses: sum of liquid then gas masses, times 1/dx^2.
-// FluidGridCPU.cpp:1399-1423 (rebuildDensity).
-__global__ void k_density(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
-{
-    dependent_start();
-    FC_VEC_TILE_PROLOGUE
-    const double inv_area = 1.0 / (g.dx * g.dx);
-    const int W = g.W, H = g.H, components = g.components;
-    const double* const* __restrict__ masses = g.masses;
-    double* __restrict__ density = g.density;
-#pragma unroll
-    for (int k = 0; k < kVecCells; ++k)
-    {
-        const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
-        if (x >= W || y >= H)
-            continue;
-        const long long i = (long long)y * W + x;
-        double total = 0.0;
-        for (int m = 0; m < components; ++m)
-            total += masses[m][i];
-        density[i] = total * inv_area;
-    }
-}
-
-// Face weights 2/(rho_a + rho_b), zero on walls and around solid cells.
-// FluidGridCPU.cpp:1154-1205 (rebuildPressureCoefficients).
+// Face weights 2/(rho_a + rho_b), zero on walls and around solid cells
+// (FluidGridCPU.cpp:1154-1205, rebuildPressureCoefficients). A cell's density is the sum of its
+// component masses, liquid then gas, times 1/dx^2 (:1399-1423, rebuildDensity); each thread forms
+// those of its cell and of the two beyond its faces (two of the three reads of a mass hit L1).
 template <typename T> __global__ void k_coefficients(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
     FC_VEC_TILE_PROLOGUE
-    const double* __restrict__ density = g.density;
+    const double inv_area = 1.0 / (g.dx * g.dx);
+    const int W = g.W, H = g.H, S = g.S, components = g.components;
+    const double* const* __restrict__ masses = g.masses;
     T* __restrict__ right = static_cast<T*>(g.lev[0].right);
     T* __restrict__ down = static_cast<T*>(g.lev[0].down);
-    const int W = g.W, H = g.H, S = g.S;
     const unsigned char* __restrict__ solid_mask = g.solid;
     unsigned char* __restrict__ air = g.air;
     const double* __restrict__ fraction = g.fraction;
     auto solid_at = [&](int sx, int sy) { return solid_mask && solid_mask[(long long)sy * W + sx]; };
-#pragma unroll
+#pragma unroll 4
     for (int k = 0; k < kVecCells; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
@@ -152,13 +131,21 @@ template <typename T> __global__ void k_coefficients(const GridDesc* __restrict_
         const bool solid = solid_at(x, y);
         if (air)
             air[c] = !solid && !(fraction[c] > 0.5); // FluidGridCPU.cpp:1321-1322: liquid is f > 0.5
-        double wr = 0.0, wd = 0.0;
-        if (x + 1 < W && !solid && !solid_at(x + 1, y))
-            wr = 2.0 / (density[c] + density[c + 1]);
-        if (y + 1 < H && !solid && !solid_at(x, y + 1))
-            wd = 2.0 / (density[c] + density[c + W]);
-        right[i] = T(wr);
-        down[i] = T(wd);
+        const bool open_r = x + 1 < W && !solid && !solid_at(x + 1, y);
+        const bool open_d = y + 1 < H && !solid && !solid_at(x, y + 1);
+        const long long cr = open_r ? c + 1 : c, cd = open_d ? c + W : c;
+        double own = 0.0, beside = 0.0, below = 0.0;
+        for (int m = 0; m < components; ++m)
+        {
+            const double* __restrict__ mass = masses[m];
+            own += mass[c];
+            beside += mass[cr];
+            below += mass[cd];
+        }
+        // Each density rounded as the reference stores it (no fused multiply-add).
+        const double rho = __dmul_rn(own, inv_area);
+        right[i] = T(open_r ? 2.0 / __dadd_rn(rho, __dmul_rn(beside, inv_area)) : 0.0);
+        down[i] = T(open_d ? 2.0 / __dadd_rn(rho, __dmul_rn(below, inv_area)) : 0.0);
     }
 }
 

@@ -13,7 +13,7 @@
 //  * The restriction's sums along x come from the residual registers; the coarse level's lanes
 //    sum them along y straight into their right-hand side registers.
 //  * The coarsest solve is one matrix product: its mean removals are folded into the inverse when
-//    it is built (k_coarse_inverse).
+//    it is built (k_rebuild_tail).
 //  * The layout and the transfer weights come in one host-built block (TailTable).
 //
 // Measured with fc_time_kernel on a 512 x 512 grid (levels 32 x 32, 16 x 16, 8 x 8), before this
@@ -617,9 +617,12 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
 }
 
 // ------------------------------------------------------------------------------------------
-// The coarsest level's explicit inverse
+// Rebuild of the tail's levels and of the coarsest level's explicit inverse
 // ------------------------------------------------------------------------------------------
 
+// One CTA per grid. The levels from the tail on hold a few thousand cells, less than a launch's worth
+// of work each: they are rebuilt here, a barrier between levels, and the coarsest inverse after them.
+//
 // Dense pinned operator of the coarsest level and its inverse in FP64; one CTA per grid
 // (PressureMultigrid.cpp:300-345, factorCoarsest). The first open cell is pinned (the reference
 // pins cell 0; with no obstacle the two are the same), Dirichlet air pins none. Gauss-Jordan
@@ -636,11 +639,18 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
 // column in shared memory, double-buffered, so it costs one barrier and one division deep.
 constexpr int kCoarseThreads = 8 * kMaxCoarse;
 
-template <typename T> __global__ void __launch_bounds__(kCoarseThreads) k_coarse_inverse(const GridDesc* __restrict__ grids)
+template <typename T> __global__ void __launch_bounds__(kCoarseThreads) k_rebuild_tail(const GridDesc* __restrict__ grids)
 {
     dependent_start();
     const GridDesc& g = grids[blockIdx.x];
     const int level = g.levels - 1;
+    for (int i = g.tail; i < level; ++i)
+    {
+        const int w = g.lev[i + 1].w, cells = w * g.lev[i + 1].h;
+        for (int q = threadIdx.x; q < cells; q += kCoarseThreads)
+            rebuild_cell<T>(g, i, q % w, q / w);
+        __syncthreads();
+    }
     const LevelDesc& l = g.lev[level];
     const int cells = l.w * l.h;
     constexpr int N = kMaxCoarse, E = kMaxCoarse / 8;
