@@ -93,7 +93,7 @@ __global__ void k_advect_velocity(const GridDesc* __restrict__ grids, const Tile
     const T* __restrict__ v = static_cast<const T*>(g.v);
     const int W = g.W, H = g.H;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < kShortCells; ++k)
     {
         const int i = t.x0 + tx + 32 * (k & 1), j = t.y0 + ty + 8 * (k >> 1);
         if (i <= W && j < H)
@@ -132,7 +132,7 @@ __global__ void k_advect_cells(const GridDesc* __restrict__ grids, const Tile* _
     const T* __restrict__ v = static_cast<const T*>(g.v);
     const int W = g.W, H = g.H;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < kShortCells; ++k)
     {
         const int i = t.x0 + tx + 32 * (k & 1), j = t.y0 + ty + 8 * (k >> 1);
         if (i >= W || j >= H)

@@ -23,13 +23,31 @@ namespace fc
 
 constexpr int kMaxLevels = 16;
 constexpr int kPadX = 2;   // column of x = 0 inside a padded row
-// Tiles of the fine-level vector kernels: 64 x 64 cells, 256 threads. Thread (lane, warp) covers
-// columns lane and lane + 32 of rows warp + 8m (kVecCells cells), or, in the strip kernels,
-// columns 2 lane and 2 lane + 1 of rows 8 warp .. 8 warp + 7.
+// Tiles of the fine-level vector kernels: 64 columns and 4 CELLS rows, 256 threads. Thread (lane,
+// warp) covers columns lane and lane + 32 of rows warp + 8m (CELLS cells), or, in the strip kernels,
+// columns 2 lane and 2 lane + 1 of CELLS / 2 rows. A grid takes tall tiles (16 cells a thread) or
+// short ones (4), see vec_cells.
 constexpr int kVecTileX = 64;
-constexpr int kVecTileY = 64;
 constexpr int kVecThreads = 256;
-constexpr int kVecCells = 16;
+constexpr int kTallCells = 16;
+constexpr int kShortCells = 4;
+constexpr int kTallTileY = 4 * kTallCells;
+constexpr int kShortTileY = 4 * kShortCells;
+
+// Cells per thread of a W x H grid's vector tiles. A thread's cells are a serial chain of load
+// latencies (the direction operator's passes of two rows most of all), so a grid whose tall tiles
+// leave SMs without one takes short tiles, which spread it over four times the CTAs; once every SM
+// has a tall tile, the per-tile reductions cost more than that gains. Whole projections with tall
+// and with short tiles, FP32: 512 x 512 (64 tall tiles) 3491 -> 3089 us, 704 x 704 (121) 3625 ->
+// 3465, 768 x 768 (144) 4774 -> 4493, 832 x 832 (169) 4983 -> 5067, 1024 x 1024 (256) 4963 -> 5319;
+// FP64: 704 x 704 3973 -> 3940, 832 x 832 5337 -> 5528. The rule looks at the grid alone, so a
+// grid's sums do not depend on what else is in its batch.
+constexpr int kShortTileLimit = 148; // tall tiles, one per SM
+inline int vec_cells(int W, int H)
+{
+    const long long tall = (long long)((W + kVecTileX - 1) / kVecTileX) * ((H + kTallTileY - 1) / kTallTileY);
+    return tall <= kShortTileLimit ? kShortCells : kTallCells;
+}
 
 __host__ __device__ inline int padded_stride(int w) { return ((w + 3) + 7) / 8 * 8; }
 __host__ __device__ inline long long padded_index(int S, int x, int y) { return (long long)(y + 1) * S + x + kPadX; }

@@ -149,6 +149,23 @@ void launch_dependent(const char* name, void (*kernel)(Params...), Blocks blocks
 #define FC_LAUNCH_DEP(kernel, blocks, threads, smem, stream, ...) \
     launch_dependent(#kernel, kernel, (blocks), (threads), (smem), (stream), __VA_ARGS__)
 
+// Launches a vector kernel (a template on CELLS) over the plan's tall and short tiles; `launch` is
+// FC_LAUNCH or FC_LAUNCH_DEP, and a kernel name with commas goes in parentheses.
+#define FC_LAUNCH_VEC(launch, kernel, p, stream, ...)                                                                 \
+    do                                                                                                               \
+    {                                                                                                                \
+        if ((p).vec[0].count > 0)                                                                                    \
+        {                                                                                                            \
+            constexpr int CELLS = ::fc::kTallCells;                                                                  \
+            launch(kernel, (p).vec[0].count, ::fc::kVecThreads, 0, stream, (p).d_desc, (p).at((p).vec[0]), ##__VA_ARGS__); \
+        }                                                                                                            \
+        if ((p).vec[1].count > 0)                                                                                    \
+        {                                                                                                            \
+            constexpr int CELLS = ::fc::kShortCells;                                                                 \
+            launch(kernel, (p).vec[1].count, ::fc::kVecThreads, 0, stream, (p).d_desc, (p).at((p).vec[1]), ##__VA_ARGS__); \
+        }                                                                                                            \
+    } while (0)
+
 int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // ------------------------------------------------------------------------------------------
@@ -572,7 +589,7 @@ size_t allocate_grid(Grid& g, bool allocate = true)
     d.dx = g.dx;
     d.levels = int(g.levels.size());
     d.tail = g.tail;
-    d.vec_tiles = ceil_div(W, kVecTileX) * ceil_div(H, kVecTileY);
+    d.vec_tiles = ceil_div(W, kVecTileX) * ceil_div(H, 4 * vec_cells(W, H));
     // The level-0 post kernel writes one (sum z, sum r z) pair per tile: slots for the most
     // tiles any region shape gives (two pairs to a double4 slot).
     const TileSizes ts = tile_sizes(g.precision, kShapeShort);
@@ -809,6 +826,7 @@ __global__ void k_init_states(const GridDesc* grids, int n, const ProjectParams*
 }
 
 // Open (non-solid) cells define the mean-free subspace of the solve.
+template <int CELLS>
 __global__ void __launch_bounds__(kVecThreads) k_count_open(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
@@ -818,7 +836,7 @@ __global__ void __launch_bounds__(kVecThreads) k_count_open(const GridDesc* __re
         return;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     double open = 0.0;
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < CELLS; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x >= g.W || y >= g.H)
@@ -864,7 +882,7 @@ template <typename T> __global__ void k_gravity(const GridDesc* grids, const Til
     const GridDesc& g = grids[t.grid];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     T* v = static_cast<T*>(g.v);
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < kShortCells; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x >= g.W || y >= g.H || y == 0)
@@ -907,7 +925,7 @@ __global__ void k_air_faces_init(const GridDesc* grids, const Tile* tiles, unsig
     const Tile t = tiles[blockIdx.x];
     const GridDesc& g = grids[t.grid];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < kShortCells; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x <= g.W && y < g.H)
@@ -966,7 +984,7 @@ __global__ void k_air_faces_extend(const GridDesc* grids, const Tile* tiles, uns
     const Tile t = tiles[blockIdx.x];
     const GridDesc& g = grids[t.grid];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < kShortCells; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x <= g.W && y < g.H)
@@ -981,7 +999,7 @@ __global__ void k_classify(const GridDesc* grids, const Tile* tiles, const doubl
     const Tile t = tiles[blockIdx.x];
     const GridDesc& g = grids[t.grid];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < kShortCells; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x >= g.W || y >= g.H)
@@ -1015,8 +1033,12 @@ struct Plan
     SolveState* d_states = nullptr;
     SolveState* h_states = nullptr;
     int* d_body_count = nullptr;
-    Range vec;
-    Range faces; // tiles over the (W+1) x (H+1) face index space
+    // Vector tiles of the grids that take tall ones ([0]) and short ones ([1]); consecutive, so that
+    // vec_all covers both.
+    Range vec[2];
+    Range vec_all;
+    Range cells; // short tiles over every grid's cells
+    Range faces; // short tiles over the (W+1) x (H+1) face index space
     Range pre[kMaxLevels];
     Range post[kMaxLevels];
     // Region shape (RegionShape) of each level's pre- and post-smoothing kernels.
@@ -1129,15 +1151,24 @@ std::unique_ptr<Plan> make_plan(const std::vector<Grid*>& grids, cudaStream_t st
         body();
         r.count = int(tiles.size()) - r.offset;
     };
-    add(plan->vec, [&]
+    for (int shape = 0; shape < 2; ++shape)
+        add(plan->vec[shape], [&]
+        {
+            const int cells = shape == 0 ? kTallCells : kShortCells;
+            for (int i = 0; i < n; ++i)
+                if (vec_cells(grids[i]->W, grids[i]->H) == cells)
+                    append_tiles(tiles, i, grids[i]->W, grids[i]->H, kVecTileX, 4 * cells);
+        });
+    plan->vec_all = {plan->vec[0].offset, plan->vec[0].count + plan->vec[1].count};
+    add(plan->cells, [&]
     {
         for (int i = 0; i < n; ++i)
-            append_tiles(tiles, i, grids[i]->W, grids[i]->H, kVecTileX, kVecTileY);
+            append_tiles(tiles, i, grids[i]->W, grids[i]->H, kVecTileX, kShortTileY);
     });
     add(plan->faces, [&]
     {
         for (int i = 0; i < n; ++i)
-            append_tiles(tiles, i, grids[i]->W + 1, grids[i]->H + 1, kVecTileX, kVecTileY);
+            append_tiles(tiles, i, grids[i]->W + 1, grids[i]->H + 1, kVecTileX, kShortTileY);
     });
     for (Grid* g : grids)
     {
@@ -1223,7 +1254,7 @@ std::unique_ptr<Plan> make_plan(const std::vector<Grid*>& grids, cudaStream_t st
 template <typename T> void launch_rebuild(Plan& p)
 {
     cudaStream_t s = p.stream;
-    FC_LAUNCH_DEP(k_coefficients<T>, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec));
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_coefficients<T, CELLS>), p, s);
     // Level by level: a coarse level follows from the finer one's weights and, under Dirichlet air,
     // its held cells from the finer level's inverse diagonal.
     for (int l = 0; l < p.max_tail; ++l)
@@ -1343,7 +1374,7 @@ template <typename T> void launch_precondition(Plan& p, bool use_mg)
     cudaStream_t s = p.stream;
     if (!use_mg)
     {
-        FC_LAUNCH_DEP(k_precondition_diagonal<T>, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec));
+        FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_precondition_diagonal<T, CELLS>), p, s);
         return;
     }
     for (int l = 0; l < p.max_tail; ++l)
@@ -1356,10 +1387,10 @@ template <typename T> void launch_precondition(Plan& p, bool use_mg)
 template <typename T> void launch_iteration(Plan& p, bool use_mg, int parity)
 {
     cudaStream_t s = p.stream;
-    FC_LAUNCH_DEP(k_direction_operator<T>, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec), parity);
-    FC_LAUNCH_DEP(k_update<T>, std::min(p.vec.count, kUpdateCtasPerSm * sm_count()), kVecThreads, 0, s, p.d_desc,
-        p.at(p.vec), p.vec.count, parity);
-    FC_LAUNCH_DEP(k_true_residual<T>, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec), 0);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_direction_operator<T, CELLS>), p, s, parity);
+    FC_LAUNCH_DEP(k_update<T>, std::min(p.vec_all.count, kUpdateCtasPerSm * sm_count()), kVecThreads, 0, s, p.d_desc,
+        p.at(p.vec_all), p.vec_all.count, parity);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_true_residual<T, CELLS>), p, s, 0);
     launch_precondition<T>(p, use_mg);
 }
 
@@ -1369,12 +1400,12 @@ template <typename T> void launch_setup(Plan& p, bool use_mg)
     cudaStream_t s = p.stream;
     // The first launch follows a copy (or starts the graph); the others follow a kernel.
     FC_LAUNCH(k_init_states, ceil_div(p.n(), 128), 128, 0, s, p.d_desc, p.n(), p.d_params, p.d_body_count);
-    FC_LAUNCH_DEP(k_count_open, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec));
-    FC_LAUNCH_DEP(k_rhs<T>, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec));
-    FC_LAUNCH_DEP(k_rhs_stats<T>, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec));
-    FC_LAUNCH_DEP(k_warm_start, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec));
-    FC_LAUNCH_DEP(k_remove_pressure_mean, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec));
-    FC_LAUNCH_DEP(k_true_residual<T>, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec), 1);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, k_count_open<CELLS>, p, s);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_rhs<T, CELLS>), p, s);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_rhs_stats<T, CELLS>), p, s);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, k_warm_start<CELLS>, p, s);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, k_remove_pressure_mean<CELLS>, p, s);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_true_residual<T, CELLS>), p, s, 1);
     launch_precondition<T>(p, use_mg);
 }
 
@@ -1384,11 +1415,11 @@ template <typename T> void launch_finish(Plan& p)
     cudaStream_t s = p.stream;
     // The first launch follows the loop (a conditional node in the graph); the others follow a
     // kernel.
-    FC_LAUNCH(k_flush_pressure<T>, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec));
-    FC_LAUNCH_DEP(k_pressure_sum, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec));
-    FC_LAUNCH_DEP(k_velocity_update<T>, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec));
-    FC_LAUNCH_DEP(k_remove_pressure_mean, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec));
-    FC_LAUNCH_DEP(k_divergence<T>, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec));
+    FC_LAUNCH(k_flush_pressure<T>, p.vec_all.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec_all));
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, k_pressure_sum<CELLS>, p, s);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_velocity_update<T, CELLS>), p, s);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, k_remove_pressure_mean<CELLS>, p, s);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_divergence<T, CELLS>), p, s);
     FC_LAUNCH_DEP(k_gather_states, ceil_div(p.n(), 128), 128, 0, s, p.d_desc, p.n(), p.d_states);
 }
 
@@ -1797,7 +1828,7 @@ void advect_semi_lagrangian(Grid& g, double dt, bool wait)
         for (int k = 0; k < fields; ++k)
         {
             double* field = k == 0 ? g.fraction : g.masses + size_t(k - 1) * g.cells;
-            FC_LAUNCH(k_advect_cells<T>, p.vec.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec), scale, half, field,
+            FC_LAUNCH(k_advect_cells<T>, p.cells.count, kVecThreads, 0, s, p.d_desc, p.at(p.cells), scale, half, field,
                 g.staging);
             check(cudaMemcpyAsync(field, g.staging, g.cells * sizeof(double), cudaMemcpyDeviceToDevice, s), "advect");
         }
@@ -2413,7 +2444,7 @@ double time_kernel(Grid& g, int kernel, int repeats)
             {
             case 0: launch_smooth<T>(p, 0, true, false, p.stream); break;
             case 1: launch_smooth<T>(p, 0, false, false, p.stream); break;
-            case 2: FC_LAUNCH(k_direction_operator<T>, p.vec.count, kVecThreads, 0, p.stream, p.d_desc, p.at(p.vec), 0); break;
+            case 2: FC_LAUNCH_VEC(FC_LAUNCH, (k_direction_operator<T, CELLS>), p, p.stream, 0); break;
             default: launch_tail<T>(p, false, p.stream); break;
             }
         };
@@ -2931,7 +2962,7 @@ void apply_gravity(Grid& g, double dt, bool wait)
     dispatch(g.precision, [&](auto zero)
     {
         using T = decltype(zero);
-        FC_LAUNCH(k_gravity<T>, p.vec.count, kVecThreads, 0, p.stream, p.d_desc, p.at(p.vec), g.gravity_y * dt);
+        FC_LAUNCH(k_gravity<T>, p.cells.count, kVecThreads, 0, p.stream, p.d_desc, p.at(p.cells), g.gravity_y * dt);
     });
     if (wait)
         check(cudaStreamSynchronize(p.stream), "gravity");
@@ -3649,7 +3680,7 @@ int fc_max_divergence(fc_grid* grid, double* out)
         fc::dispatch(g.precision, [&](auto zero)
         {
             using T = decltype(zero);
-            FC_LAUNCH(fc::k_divergence<T>, p.vec.count, fc::kVecThreads, 0, p.stream, p.d_desc, p.at(p.vec));
+            FC_LAUNCH_VEC(FC_LAUNCH, (fc::k_divergence<T, CELLS>), p, p.stream);
         });
         fc::SolveState s;
         check(cudaMemcpyAsync(&s, g.desc.state, sizeof(s), cudaMemcpyDeviceToHost, p.stream), "divergence");
@@ -3667,7 +3698,7 @@ int fc_classify(fc_grid* grid, unsigned char* mask)
         Grid& g = grid->impl;
         fc::require_uploaded(g);
         fc::Plan& p = fc::single_plan(g);
-        FC_LAUNCH(fc::k_classify, p.vec.count, fc::kVecThreads, 0, p.stream, p.d_desc, p.at(p.vec), g.fraction, g.mask);
+        FC_LAUNCH(fc::k_classify, p.cells.count, fc::kVecThreads, 0, p.stream, p.d_desc, p.at(p.cells), g.fraction, g.mask);
         check(cudaMemcpyAsync(mask, g.mask, g.cells, cudaMemcpyDeviceToHost, p.stream), "classify");
         check(cudaStreamSynchronize(p.stream), "classify");
     });

@@ -42,7 +42,7 @@ __device__ __forceinline__ void finish_preconditioner(SolveState& s, double sum_
 }
 
 // Diagonal (Jacobi) preconditioner: z = (r - mean r) / diag. FluidGridCPU.cpp:1691-1698.
-template <typename T>
+template <typename T, int CELLS>
 __global__ void __launch_bounds__(kVecThreads) k_precondition_diagonal(const GridDesc* grids, const Tile* tiles)
 {
     allow_dependents();
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kVecThreads) k_precondition_diagonal(const Gri
     T* z = static_cast<T*>(g.z);
     const double mean_r = s.mean_r;
     double sz = 0.0, srz = 0.0;
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < CELLS; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x >= g.W || y >= g.H)

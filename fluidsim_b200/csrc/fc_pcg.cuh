@@ -1,8 +1,9 @@
 // Fine-level PCG kernels of the UniformCUDA projection.
 //
 // Every kernel takes the grid descriptors and a tile table, so one launch serves one grid or a
-// batch of independent grids of uneven sizes (each CTA looks up its grid). A tile is 32 x 32
-// cells worked by 256 threads, 4 rows each. Reductions are folded in FP64: each CTA writes one
+// batch of independent grids of uneven sizes (each CTA looks up its grid). A tile is 64 columns and
+// 4 CELLS rows (64 or 16, by the grid's size; vec_cells), worked by 256 threads of CELLS cells each.
+// Reductions are folded in FP64: each CTA writes one
 // partial and the last CTA of a grid to arrive folds them in tile order, so results do not
 // depend on which other grids share the launch.
 //
@@ -107,7 +108,7 @@ __device__ __forceinline__ bool held_at(const unsigned char* __restrict__ solid,
 // (FluidGridCPU.cpp:1154-1205, rebuildPressureCoefficients). A cell's density is the sum of its
 // component masses, liquid then gas, times 1/dx^2 (:1399-1423, rebuildDensity); each thread forms
 // those of its cell and of the two beyond its faces (two of the three reads of a mass hit L1).
-template <typename T> __global__ void k_coefficients(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
+template <typename T, int CELLS> __global__ void k_coefficients(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
     FC_VEC_TILE_PROLOGUE
@@ -121,7 +122,7 @@ template <typename T> __global__ void k_coefficients(const GridDesc* __restrict_
     const double* __restrict__ fraction = g.fraction;
     auto solid_at = [&](int sx, int sy) { return solid_mask && solid_mask[(long long)sy * W + sx]; };
 #pragma unroll 4
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < CELLS; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x >= W || y >= H)
@@ -184,7 +185,7 @@ __device__ __forceinline__ void cell_faces(T* __restrict__ u, T* __restrict__ v,
 
 // b = -(du + dv)/dx * dx^2/dt with closed faces zeroed; sums b over open cells.
 // FluidGridCPU.cpp:1050-1083.
-template <typename T> __global__ void __launch_bounds__(kVecThreads) k_rhs(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
+template <typename T, int CELLS> __global__ void __launch_bounds__(kVecThreads) k_rhs(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
     FC_VEC_TILE_PROLOGUE
@@ -199,7 +200,7 @@ template <typename T> __global__ void __launch_bounds__(kVecThreads) k_rhs(const
     double* __restrict__ rhs = g.b;
     double sum = 0.0;
 #pragma unroll
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < CELLS; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x >= W || y >= H)
@@ -223,7 +224,7 @@ template <typename T> __global__ void __launch_bounds__(kVecThreads) k_rhs(const
 }
 
 // max |b - mean| and sum (b - mean)^2; decides the early exit (FluidGridCPU.cpp:1731-1740).
-template <typename T> __global__ void __launch_bounds__(kVecThreads) k_rhs_stats(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
+template <typename T, int CELLS> __global__ void __launch_bounds__(kVecThreads) k_rhs_stats(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
     FC_VEC_TILE_PROLOGUE
@@ -234,7 +235,7 @@ template <typename T> __global__ void __launch_bounds__(kVecThreads) k_rhs_stats
     const double* __restrict__ rhs = g.b;
     double mx = 0.0, sq = 0.0;
 #pragma unroll
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < CELLS; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x >= W || y >= H || held_at(solid, air, W, x, y))
@@ -264,7 +265,7 @@ template <typename T> __global__ void __launch_bounds__(kVecThreads) k_rhs_stats
 
 // Warm start p = 2p - p_prev, or clear both when no solve is needed; sums the prediction.
 // FluidGridCPU.cpp:1731-1753.
-__global__ void __launch_bounds__(kVecThreads) k_warm_start(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
+template <int CELLS> __global__ void __launch_bounds__(kVecThreads) k_warm_start(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
     FC_VEC_TILE_PROLOGUE
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(kVecThreads) k_warm_start(const GridDesc* __re
     double* __restrict__ p_prev = g.p_prev;
     double sum = 0.0;
 #pragma unroll
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < CELLS; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x >= W || y >= H)
@@ -303,7 +304,7 @@ __global__ void __launch_bounds__(kVecThreads) k_warm_start(const GridDesc* __re
 }
 
 // Pressure sum for the final mean removal.
-__global__ void __launch_bounds__(kVecThreads) k_pressure_sum(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
+template <int CELLS> __global__ void __launch_bounds__(kVecThreads) k_pressure_sum(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
     FC_VEC_TILE_PROLOGUE
@@ -315,7 +316,7 @@ __global__ void __launch_bounds__(kVecThreads) k_pressure_sum(const GridDesc* __
     const double* __restrict__ p = g.p;
     double sum = 0.0;
 #pragma unroll
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < CELLS; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x >= W || y >= H || held_at(solid, air, W, x, y))
@@ -331,7 +332,7 @@ __global__ void __launch_bounds__(kVecThreads) k_pressure_sum(const GridDesc* __
 }
 
 // p -= mean_p over open cells (FluidGridCPU.cpp:1466-1474, removeMean).
-__global__ void k_remove_pressure_mean(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
+template <int CELLS> __global__ void k_remove_pressure_mean(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
     FC_VEC_TILE_PROLOGUE
@@ -343,7 +344,7 @@ __global__ void k_remove_pressure_mean(const GridDesc* __restrict__ grids, const
     const unsigned char* __restrict__ air = g.air;
     double* __restrict__ p = g.p;
 #pragma unroll
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < CELLS; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x >= W || y >= H)
@@ -381,7 +382,7 @@ __device__ __forceinline__ double apply_cell_fp64_pending(const T* right, const 
 // True residual r = (b - mean b) - A p in FP64, stored in the working type, with its stats.
 // `initial` selects the solve's first residual (FluidGridCPU.cpp:1754-1757) versus the
 // convergence check inside the loop (:1795-1804).
-template <typename T>
+template <typename T, int CELLS>
 __global__ void __launch_bounds__(kVecThreads) k_true_residual(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles, int initial)
 {
     allow_dependents();
@@ -405,7 +406,7 @@ __global__ void __launch_bounds__(kVecThreads) k_true_residual(const GridDesc* _
     const double alpha0 = s.alpha_pending;
     double sum = 0.0, mx = 0.0, sq = 0.0;
 #pragma unroll
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < CELLS; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x >= W || y >= H)
@@ -472,20 +473,21 @@ template <> struct VecPair<double>
     using type = double2;
 };
 
-// d = (z - mean z) + beta d_old; q = A d; d.q through the grid's reduction. Warp w handles rows
-// 8w .. 8w + 7 of the tile's 64 columns (lane = column pair) in four passes of two rows: all
+// d = (z - mean z) + beta d_old; q = A d; d.q through the grid's reduction. Warp w handles
+// CELLS / 2 rows of the tile's 64 columns (lane = column pair) in passes of two rows: all
 // loads of a pass (four rows of z and d, two rows of weights) are issued first, then the
 // directions and the operator are formed in registers; horizontal neighbours across pairs are
 // warp shuffles, and lanes 0 and 31 fetch the columns just outside the warp. At 64 registers
 // four CTAs fit an SM in FP32, which hides more load latency than passes of four rows at 80
 // registers and three CTAs (31.5 -> 30.2 us at 2048 x 2048).
 // Operator: FluidGridCPU.cpp:1507-1598.
-template <typename T>
+template <typename T, int CELLS>
 __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? 4 : 1)
     k_direction_operator(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles, int parity)
 {
     using P = typename VecPair<T>::type;
     constexpr int R = 2;
+    constexpr int ROWS = CELLS / 2; // of each warp
     allow_dependents();
     const Tile t = tiles[blockIdx.x];
     const GridDesc& g = grids[t.grid];
@@ -510,12 +512,12 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? 4 : 1)
     const bool edge = (lane == 0 && cols) || (lane == 31 && gx + 2 + kPadX < S);
     P up_w = P{};
     if (cols)
-        up_w = *reinterpret_cast<const P*>(down + padded_index(S, gx, t.y0 + 8 * warp - 1));
+        up_w = *reinterpret_cast<const P*>(down + padded_index(S, gx, t.y0 + ROWS * warp - 1));
     double dot = 0.0;
 #pragma unroll 1
-    for (int pass = 0; pass < 8 / R; ++pass)
+    for (int pass = 0; pass < ROWS / R; ++pass)
     {
-        const int y0 = t.y0 + 8 * warp + R * pass;
+        const int y0 = t.y0 + ROWS * warp + R * pass;
         P zz[R + 2], dd0[R + 2], w[R], dn[R];
         T ez[R], ed[R], ew[R];
 #pragma unroll
@@ -814,7 +816,7 @@ template <typename T> __global__ void __launch_bounds__(kVecThreads) k_flush_pre
 
 // u -= (dp/dx) dt w on open interior faces; each cell updates its left and upper face.
 // FluidGridCPU.cpp:1098-1118.
-template <typename T> __global__ void k_velocity_update(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
+template <typename T, int CELLS> __global__ void k_velocity_update(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
     FC_VEC_TILE_PROLOGUE
@@ -828,7 +830,7 @@ template <typename T> __global__ void k_velocity_update(const GridDesc* __restri
     const T* __restrict__ down = static_cast<const T*>(g.lev[0].down);
     const double* __restrict__ p = g.p;
 #pragma unroll
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < CELLS; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x >= W || y >= H)
@@ -872,7 +874,7 @@ __device__ __forceinline__ double face_ulp(double value)
 // max |div u| (FluidGridCPU.cpp:1126-1152), its excess over the float rounding allowance of the
 // four faces (as UniformWebGPU's velocity_stats, FluidUniformWebGPUKernels.h:166-213), and the
 // sum of squares.
-template <typename T> __global__ void __launch_bounds__(kVecThreads) k_divergence(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
+template <typename T, int CELLS> __global__ void __launch_bounds__(kVecThreads) k_divergence(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
     FC_VEC_TILE_PROLOGUE
@@ -886,7 +888,7 @@ template <typename T> __global__ void __launch_bounds__(kVecThreads) k_divergenc
     double mx = 0.0, excess = 0.0, sq = 0.0;
     int nonfinite = 0;
 #pragma unroll
-    for (int k = 0; k < kVecCells; ++k)
+    for (int k = 0; k < CELLS; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x >= W || y >= H)
