@@ -1,0 +1,41 @@
+"""The viscosity V-cycle's kernels at the sizes where their tiles, rings and one-CTA levels end, against
+the FP64 restatement: variable viscosity and density, so that every coefficient differs."""
+import numpy as np
+import pytest
+
+from fluidsim_b200 import FluidGrid, FluidGridState
+
+pytestmark = pytest.mark.gpu
+
+# A single level, thin lattices, the restriction's and prolongation's 32 x 8 tiles and their
+# remainders, levels of at most and of more than one node per thread of the one-CTA cycle, and two
+# and three levels above it.
+SIZES = [(8, 8), (3, 90), (90, 3), (31, 31), (32, 33), (63, 16), (66, 65), (97, 130), (257, 66), (300, 211)]
+
+
+@pytest.mark.parametrize("precision,bound", [("fp64", 1e-10), ("fp32", 1e-3)])
+@pytest.mark.parametrize("size", SIZES, ids=lambda s: f"{s[0]}x{s[1]}")
+def test_solve_matches_restatement(oracle, size, precision, bound):
+    """FP64 to rounding and the same iteration count. FP32 within 1e-3 of scale: it stops at the same
+    1e-4 rule, where a change of rounding moves the iterate by about its own tolerance."""
+    w, h = size
+    dx, dt = 1.0 / max(w, h), 1.0 / 120.0
+    y, x = np.mgrid[0:h, 0:w]
+    share = 0.5 + 0.5 * np.sin(0.31 * x + 0.17 * y)
+    lm, gm = 900.0 * share * dx * dx, 40.0 * (1.0 - share) * dx * dx
+    rng = np.random.default_rng(w * 1000 + h)
+    u, v = rng.uniform(-1, 1, (h, w + 1)), rng.uniform(-1, 1, (h + 1, w))
+    u, v = u.astype(np.float32).astype(float), v.astype(np.float32).astype(float)
+    u[:, 0] = u[:, -1] = 0.0
+    v[0] = v[-1] = 0.0
+    g = FluidGrid(w, h, dx, precision)
+    g.configureMaterials([900.0], [40.0], [2.0], [0.01])
+    g.upload(FluidGridState(share, u, v, None, [lm], [gm]))
+    it, _ = g.applyViscosity(dt, 1e-4)
+    material = oracle.viscosity_material([lm, gm], [900.0, 40.0], [2.0, 0.01], dx)
+    expected_it, eu, ev, _ = oracle.Viscosity(w, h).solve(u, v, material, dt, dx, 1e-4)
+    s = g.download()
+    scale = max(np.abs(eu).max(), np.abs(ev).max())
+    if precision == "fp64":
+        assert it == expected_it
+    assert np.abs(s.u - eu).max() <= bound * scale and np.abs(s.v - ev).max() <= bound * scale
