@@ -135,14 +135,15 @@ struct LevelDesc
     void* sol;           // final solution of the level (level 0: the PCG vector z)
     const double* cx;    // cell centres, in fine cells
     const double* cy;
-    const Interp* px;    // fine level -> this level's coarse parent (valid for l < last)
-    const Interp* py;
-    const Gather* rx;    // coarse (l+1) cell -> fine cells of l
-    const Gather* ry;
-    // The same per coarse column / row as offset weights in the working precision
-    // (RestrictAxis<T>, fc_smooth.cuh), built by the host from rx / ry.
+    // Restriction weights per coarse column and row of the next level, in the working precision
+    // (RestrictAxis<T>, fc_smooth.cuh).
     const void* rwx;
     const void* rwy;
+    // Prolongation weights of this level's columns and rows in the working precision, on fixed
+    // coarse neighbours: cells 2m and 2m + 1 blend coarse cells m - 1, m and m, m + 1, the weight
+    // belonging to the second (prolong_weights in the engine, from the interpolation tables).
+    const void* pwx;
+    const void* pwy;
 };
 
 struct GridDesc

@@ -182,7 +182,7 @@ struct HostLevel
     std::vector<unsigned char> pwx, pwy; // px, py as prolong_weights of the grid's precision
 };
 
-// Offset weights of a restriction table (what restrict_axis forms on the device).
+// Offset weights of a restriction table.
 template <typename T> std::vector<unsigned char> restrict_weights(const std::vector<Gather>& table)
 {
     std::vector<unsigned char> bytes(table.size() * sizeof(RestrictAxis<T>));
@@ -202,7 +202,7 @@ template <typename T> std::vector<unsigned char> restrict_weights(const std::vec
     return bytes;
 }
 
-// Prolongation weights on fixed coarse neighbours (the tail, fc_tail.cuh): fine cell f blends coarse cells
+// Prolongation weights on fixed coarse neighbours (LevelDesc::pwx): fine cell f blends coarse cells
 // s = f / 2 - 1 + f % 2 and s + 1 (either may lie outside the level, clamped). The table's clamped
 // entries name s + 1 as their first cell with weight zero: that is weight one on the second.
 template <typename T> std::vector<unsigned char> prolong_weights(const std::vector<Interp>& table)
@@ -629,8 +629,8 @@ size_t allocate_grid(Grid& g, bool allocate = true)
     add((void**)&g.air, g.cells);
     add((void**)&g.air_faces, g.faces_u + g.faces_v);
     add((void**)&d.lev[0].pre, padded0 * elem);
-    std::vector<void*> cx(g.levels.size()), cy(g.levels.size()), px(g.levels.size()), py(g.levels.size()),
-        rx(g.levels.size()), ry(g.levels.size()), rwx(g.levels.size()), rwy(g.levels.size());
+    std::vector<void*> cx(g.levels.size()), cy(g.levels.size()), rwx(g.levels.size()), rwy(g.levels.size()),
+        pwx(g.levels.size()), pwy(g.levels.size());
     for (size_t l = 0; l < g.levels.size(); ++l)
     {
         const HostLevel& L = g.levels[l];
@@ -660,10 +660,6 @@ size_t allocate_grid(Grid& g, bool allocate = true)
         add(&cy[l], L.cy.size() * sizeof(double));
         if (l + 1 < g.levels.size())
         {
-            add(&px[l], L.px.size() * sizeof(Interp));
-            add(&py[l], L.py.size() * sizeof(Interp));
-            add(&rx[l], L.rx.size() * sizeof(Gather));
-            add(&ry[l], L.ry.size() * sizeof(Gather));
             HostLevel& H = g.levels[l];
             H.rwx = g.elem == 8 ? restrict_weights<double>(L.rx) : restrict_weights<float>(L.rx);
             H.rwy = g.elem == 8 ? restrict_weights<double>(L.ry) : restrict_weights<float>(L.ry);
@@ -671,6 +667,8 @@ size_t allocate_grid(Grid& g, bool allocate = true)
             add(&rwy[l], H.rwy.size());
             H.pwx = g.elem == 8 ? prolong_weights<double>(L.px) : prolong_weights<float>(L.px);
             H.pwy = g.elem == 8 ? prolong_weights<double>(L.py) : prolong_weights<float>(L.py);
+            add(&pwx[l], H.pwx.size());
+            add(&pwy[l], H.pwy.size());
         }
     }
     // TMA maps: per level, kShapes region shapes, kMapsPerSet maps of 128 bytes.
@@ -700,18 +698,14 @@ size_t allocate_grid(Grid& g, bool allocate = true)
         ld.cy = static_cast<const double*>(cy[l]);
         if (l + 1 < g.levels.size())
         {
-            check(cudaMemcpyAsync(px[l], L.px.data(), L.px.size() * sizeof(Interp), cudaMemcpyHostToDevice, g.stream), "tables");
-            check(cudaMemcpyAsync(py[l], L.py.data(), L.py.size() * sizeof(Interp), cudaMemcpyHostToDevice, g.stream), "tables");
-            check(cudaMemcpyAsync(rx[l], L.rx.data(), L.rx.size() * sizeof(Gather), cudaMemcpyHostToDevice, g.stream), "tables");
-            check(cudaMemcpyAsync(ry[l], L.ry.data(), L.ry.size() * sizeof(Gather), cudaMemcpyHostToDevice, g.stream), "tables");
-            ld.px = static_cast<const Interp*>(px[l]);
-            ld.py = static_cast<const Interp*>(py[l]);
-            ld.rx = static_cast<const Gather*>(rx[l]);
-            ld.ry = static_cast<const Gather*>(ry[l]);
             check(cudaMemcpyAsync(rwx[l], L.rwx.data(), L.rwx.size(), cudaMemcpyHostToDevice, g.stream), "tables");
             check(cudaMemcpyAsync(rwy[l], L.rwy.data(), L.rwy.size(), cudaMemcpyHostToDevice, g.stream), "tables");
             ld.rwx = rwx[l];
             ld.rwy = rwy[l];
+            check(cudaMemcpyAsync(pwx[l], L.pwx.data(), L.pwx.size(), cudaMemcpyHostToDevice, g.stream), "tables");
+            check(cudaMemcpyAsync(pwy[l], L.pwy.data(), L.pwy.size(), cudaMemcpyHostToDevice, g.stream), "tables");
+            ld.pwx = pwx[l];
+            ld.pwy = pwy[l];
         }
     }
     d.solid = nullptr;

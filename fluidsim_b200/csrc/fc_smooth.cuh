@@ -171,33 +171,12 @@ __device__ __forceinline__ void edges_clear(Edges<T, WARPS>& e)
 // One axis of the transpose-bilinear restriction for coarse cell c: the weights of fine cells
 // 2c-1, 2c, 2c+1, 2c+2 (bit p of `mask` set when fine cell 2c-1+p contributes). The table lists
 // its fine cells in ascending order, so summing by offset keeps the table's order; the host
-// checks that no entry falls outside the four offsets. The strip kernels read these per coarse
-// cell precomputed (LevelDesc::rwx, rwy); the tail forms them from its staged tables.
+// checks that no entry falls outside the four offsets (LevelDesc::rwx, rwy).
 template <typename T> struct alignas(16) RestrictAxis
 {
     T w[4];
     unsigned mask;
 };
-
-template <typename T> __device__ __forceinline__ RestrictAxis<T> restrict_axis(const Gather* table, int c)
-{
-    RestrictAxis<T> r;
-    r.mask = 0;
-    const Gather g = table[c];
-#pragma unroll
-    for (int p = 0; p < 4; ++p)
-    {
-        r.w[p] = T(0);
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-            if (e < g.count && g.index[e] == 2 * c - 1 + p)
-            {
-                r.w[p] = T(g.weight[e]);
-                r.mask |= 1u << p;
-            }
-    }
-    return r;
-}
 
 // sum over the set offsets of w[p] * v[p], accumulated in offset order from zero.
 template <typename T>

@@ -12,8 +12,7 @@
 // 2D tiles of the padded level arrays: weights, inverse diagonal, the level's vector (and for
 // the post kernel the pre-smoothed solution and the coarse solution), 72 columns x WARPS*K+1
 // rows (the strip rows and the row above, the column left of the region, rounded out to 16-byte
-// alignment); coordinates outside an array read as zero, as the padded halo does. The post kernel
-// also bulk-copies the region's rows and columns of the prolongation tables.
+// alignment); coordinates outside an array read as zero, as the padded halo does.
 #pragma once
 
 #include "fc_smooth.cuh"
@@ -33,15 +32,11 @@ template <typename T, typename W, int K, bool PRE, int WARPS = 8> struct Stage
     static constexpr size_t WB = round(size_t(BW) * BH * sizeof(W));
     static constexpr size_t VB = round(size_t(BW) * BH * sizeof(T));
     static constexpr size_t CB = PRE ? 0 : round(size_t(CBW) * CBH * sizeof(T));
-    // Post: the prolongation tables of the region's rows and columns (Interp, 16 bytes each).
-    static constexpr size_t IY = PRE ? 0 : round(size_t(WARPS) * K * sizeof(Interp));
-    static constexpr size_t IX = PRE ? 0 : round(64 * sizeof(Interp));
     // The inverse diagonal is staged rather than formed from the weights: a correctly rounded
     // FP32 reciprocal per cell cost more time (2,300 cycles a tile) than its box's copy.
     static constexpr size_t right = 0, down = WB, inv = 2 * WB, vec = 2 * WB + VB, pre = 2 * WB + 2 * VB;
     static constexpr size_t coarse = PRE ? pre : pre + VB;
-    static constexpr size_t rows = coarse + CB, cols = rows + IY;
-    static constexpr size_t bytes = cols + IX;
+    static constexpr size_t bytes = coarse + CB;
     // Bytes the boxes of one tile deliver (full boxes, zero-filled parts included).
     static constexpr unsigned tx = unsigned(2 * BW * BH * sizeof(W) + (PRE ? 2 : 3) * BW * BH * sizeof(T) +
                                             (PRE ? 0 : CBW * CBH * sizeof(T)));
@@ -79,16 +74,9 @@ __device__ __forceinline__ const void* stage_map(const char* maps, int level, in
 struct IssueArgs
 {
     const char* maps;  // the grid's tensor maps
-    const Interp* py;  // post: the level's prolongation tables
-    const Interp* px;
-    int w, h;          // the level's size
 };
 
-__device__ __forceinline__ IssueArgs issue_args(const GridDesc& g, int level)
-{
-    const LevelDesc& L = g.lev[level];
-    return IssueArgs{static_cast<const char*>(g.maps), L.py, L.px, L.w, L.h};
-}
+__device__ __forceinline__ IssueArgs issue_args(const GridDesc& g) { return IssueArgs{static_cast<const char*>(g.maps)}; }
 
 // First box column of a region whose leftmost needed padded column is v: a TMA box must start
 // at a multiple of 16 bytes, i.e. of 16 / sizeof(E) elements (4 for FP32, 8 for FP16).
@@ -109,22 +97,7 @@ __device__ __forceinline__ void stage_issue_weights(const IssueArgs& g, int leve
     // Padded coordinates: column gx + 2, row gy + 1. The region needs columns X0-1 .. X0+63 and
     // rows Y0-1 .. Y0+WARPS*K-1.
     const int bw = box_start<W>(X0 + 1), by = Y0;
-    if constexpr (!PRE)
-    {
-        // The prolongation tables of the region's in-level rows and columns, by bulk copy into
-        // slots indexed by region row / column (the kernel reads in-level slots only).
-        const int r0 = max(Y0, 0), r1 = min(Y0 + WARPS * K, g.h);
-        const int c0 = max(X0, 0), c1 = min(X0 + 64, g.w);
-        const unsigned row_bytes = r1 > r0 ? unsigned(r1 - r0) * sizeof(Interp) : 0u;
-        const unsigned col_bytes = c1 > c0 ? unsigned(c1 - c0) * sizeof(Interp) : 0u;
-        mbarrier_expect_tx(bar, S::tx + row_bytes + col_bytes);
-        if (row_bytes)
-            bulk_load(stage + S::rows + size_t(r0 - Y0) * sizeof(Interp), g.py + r0, row_bytes, bar);
-        if (col_bytes)
-            bulk_load(stage + S::cols + size_t(c0 - X0) * sizeof(Interp), g.px + c0, col_bytes, bar);
-    }
-    else
-        mbarrier_expect_tx(bar, S::tx);
+    mbarrier_expect_tx(bar, S::tx);
     tma_load_2d(stage + S::right, stage_map(g.maps, level, set, kMapRight), bw, by, bar);
     tma_load_2d(stage + S::down, stage_map(g.maps, level, set, kMapDown), bw, by, bar);
     tma_load_2d(stage + S::inv, stage_map(g.maps, level, set, kMapInverse), box_start<T>(X0 + 1), by, bar);
@@ -289,7 +262,7 @@ __global__ void __launch_bounds__(32 * WARPS, (sizeof(T) == 4 && WARPS == 8) ? 2
     // The first tile's weights stream in while the previous kernel finishes.
     if (threadIdx.x == 0 && i < count && !misplaced)
     {
-        const IssueArgs first = issue_args(grids[t.grid], level);
+        const IssueArgs first = issue_args(grids[t.grid]);
         stage_issue_weights<T, W, K, true, WARPS>(first, level, set, t.x0 - Shape::HALO, t.y0 - Shape::HALO, stage, &bar);
         stage_prefetch_data_maps<true>(first, level, set);
     }
@@ -305,7 +278,7 @@ __global__ void __launch_bounds__(32 * WARPS, (sizeof(T) == 4 && WARPS == 8) ? 2
     if (threadIdx.x == 0 && i < count)
     {
         tile_live = grids[t.grid].state->done == 0;
-        stage_issue_data<T, W, K, true, WARPS>(issue_args(grids[t.grid], level), level, set, t.x0 - Shape::HALO,
+        stage_issue_data<T, W, K, true, WARPS>(issue_args(grids[t.grid]), level, set, t.x0 - Shape::HALO,
             t.y0 - Shape::HALO, stage, &bar);
     }
     unsigned parity = 0;
@@ -340,7 +313,7 @@ __global__ void __launch_bounds__(32 * WARPS, (sizeof(T) == 4 && WARPS == 8) ? 2
         bool next_live = false;
         if (threadIdx.x == 0 && next < count)
         {
-            na = issue_args(grids[n.grid], level);
+            na = issue_args(grids[n.grid]);
             next_live = grids[n.grid].state->done == 0;
         }
         const bool ok = mbarrier_wait(&bar, parity);
@@ -494,7 +467,7 @@ __global__ void __launch_bounds__(32 * WARPS, (sizeof(T) == 4 && WARPS == 8) ? 2
     // The first tile's weights stream in while the previous kernel finishes.
     if (threadIdx.x == 0 && i < count && !misplaced)
     {
-        const IssueArgs first = issue_args(grids[t.grid], level);
+        const IssueArgs first = issue_args(grids[t.grid]);
         stage_issue_weights<T, W, K, false, WARPS>(first, level, set, t.x0 - Shape::HALO, t.y0 - Shape::HALO, stage, &bar);
         stage_prefetch_data_maps<false>(first, level, set);
     }
@@ -510,7 +483,7 @@ __global__ void __launch_bounds__(32 * WARPS, (sizeof(T) == 4 && WARPS == 8) ? 2
     if (threadIdx.x == 0 && i < count)
     {
         tile_live = grids[t.grid].state->done == 0;
-        stage_issue_data<T, W, K, false, WARPS>(issue_args(grids[t.grid], level), level, set, t.x0 - Shape::HALO,
+        stage_issue_data<T, W, K, false, WARPS>(issue_args(grids[t.grid]), level, set, t.x0 - Shape::HALO,
             t.y0 - Shape::HALO, stage, &bar);
     }
     unsigned parity = 0;
@@ -526,15 +499,24 @@ __global__ void __launch_bounds__(32 * WARPS, (sizeof(T) == 4 && WARPS == 8) ? 2
         T* const out = static_cast<T*>(Ld.sol);
         const float wscale = Ld.wscale;
         const int X0 = t.x0 - Shape::HALO, Y0 = t.y0 - Shape::HALO;
-        const int CX0 = X0 / 2 - 1, CY0 = Y0 / 2 - 1;
+        const int CX0 = X0 / 2 - 1;
         const int gx = X0 + 2 * lane;
         const bool in_a = gx >= 0 && gx < Lw, in_b = gx + 1 >= 0 && gx + 1 < Lw;
+        // Prolongation weights of the thread's columns and rows, while the tile's boxes land. Cells
+        // outside the level take those of its first or last cell; they are set to zero afterwards.
+        const T* const pwx = static_cast<const T*>(Ld.pwx);
+        const T* const pwy = static_cast<const T*>(Ld.pwy);
+        const T wxa = pwx[min(max(gx, 0), Lw - 1)], wxb = pwx[min(max(gx + 1, 0), Lw - 1)];
+        T wy[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            wy[k] = pwy[min(max(Y0 + warp * K + k, 0), Lh - 1)];
         const double mean_r = level == 0 ? state->mean_r : 0.0;
         IssueArgs na{};
         bool next_live = false;
         if (threadIdx.x == 0 && next < count)
         {
-            na = issue_args(grids[n.grid], level);
+            na = issue_args(grids[n.grid]);
             next_live = grids[n.grid].state->done == 0;
         }
         const bool ok = mbarrier_wait(&bar, parity);
@@ -558,75 +540,31 @@ __global__ void __launch_bounds__(32 * WARPS, (sizeof(T) == 4 && WARPS == 8) ? 2
                 s.b[k] = ab.y;
             }
             strip_finish<T, K>(s, level, mean_r);
-            // Add the prolonged coarse correction, in-level cells only; the tables arrived with
-            // the tile's boxes.
-            const Interp* interp_y = reinterpret_cast<const Interp*>(stage + S::rows);
-            const Interp* interp_x = reinterpret_cast<const Interp*>(stage + S::cols);
+            // Add the prolonged coarse correction. Fine cells 2m and 2m + 1 blend coarse cells m - 1, m and
+            // m, m + 1 (the region's origin is even), wherever they lie: at the level's edges the weights
+            // are 0 or 1 (prolong_weights) and the other cell is a zero of the padding. So every coarse row
+            // the warp's rows read is interpolated along x once, K / 2 + 2 rows instead of 2K, from three
+            // values a lane. (With first and second cells from 16-byte table entries per row and column, and
+            // a path of its own for warps at the edges, whole projections took 16.60 ms at 2048 x 2048 and
+            // 10.57 ms at 1920 x 1080 in mixed precision; with this 15.92 and 10.00.)
             const T* coarse = reinterpret_cast<const T*>(stage + S::coarse);
             const int coff = CX0 + 2 - box_start<T>(CX0 + 2);
-            const Interp pa = in_a ? interp_x[2 * lane] : Interp{CX0, CX0, 0.0};
-            const Interp pb = in_b ? interp_x[2 * lane + 1] : Interp{CX0, CX0, 0.0};
-            const T wxa = T(pa.weight), wxb = T(pb.weight);
-            const int fa = pa.first - CX0 + coff, sa = pa.second - CX0 + coff;
-            const int fb = pb.first - CX0 + coff, sb = pb.second - CX0 + coff;
             const int r0 = warp * K;
-            // Each coarse row the warp's rows read is interpolated along x once: K / 2 + 2 rows
-            // instead of 2K. The loads do not wait for the row tables: the box rows r0 / 2 ..
-            // r0 / 2 + K / 2 + 1 are inside the coarse box whatever the tables say.
             T xa[K / 2 + 2], xb[K / 2 + 2];
 #pragma unroll
             for (int j = 0; j < K / 2 + 2; ++j)
             {
-                const T* row = coarse + (r0 / 2 + j) * S::CBW;
-                xa[j] = prolong_lerp(wxa, row[fa], row[sa]);
-                xb[j] = prolong_lerp(wxb, row[fb], row[sb]);
+                const T* row = coarse + (r0 / 2 + j) * S::CBW + coff + lane;
+                const T v0 = row[0], v1 = row[1], v2 = row[2];
+                xa[j] = prolong_lerp(wxa, v0, v1);
+                xb[j] = prolong_lerp(wxb, v1, v2);
             }
-            Interp py[K];
-            bool regular = true;
 #pragma unroll
             for (int k = 0; k < K; ++k)
             {
-                const int gy = Y0 + r0 + k;
-                regular = regular && gy >= 0 && gy < Lh;
-                py[k] = regular ? interp_y[r0 + k] : Interp{CY0, CY0, 0.0};
-                // Away from the level's edges, fine rows 2m and 2m + 1 (the region origin is
-                // even) read coarse rows m - 1, m and m, m + 1: box rows r0 / 2 + (k + 1) / 2
-                // and the one below.
-                regular = regular && py[k].first - CY0 == r0 / 2 + (k + 1) / 2 && py[k].second == py[k].first + 1;
-            }
-            if (regular)
-            {
-#pragma unroll
-                for (int k = 0; k < K; ++k)
-                {
-                    const T wy = T(py[k].weight);
-                    const int f = (k + 1) / 2;
-                    if (in_a)
-                        s.a[k] = s.a[k] + prolong_lerp(wy, xa[f], xa[f + 1]);
-                    if (in_b)
-                        s.b[k] = s.b[k] + prolong_lerp(wy, xb[f], xb[f + 1]);
-                }
-            }
-            else
-            {
-                // Rows at the level's edges: each fine row reads its two coarse rows.
-#pragma unroll
-                for (int k = 0; k < K; ++k)
-                {
-                    const int gy = Y0 + r0 + k;
-                    if (gy < 0 || gy >= Lh)
-                        continue;
-                    const Interp q = interp_y[r0 + k];
-                    const T* top = coarse + (q.first - CY0) * S::CBW;
-                    const T* bottom = coarse + (q.second - CY0) * S::CBW;
-                    const T wy = T(q.weight);
-                    if (in_a)
-                        s.a[k] = s.a[k] + prolong_lerp(wy, prolong_lerp(wxa, top[fa], top[sa]),
-                                              prolong_lerp(wxa, bottom[fa], bottom[sa]));
-                    if (in_b)
-                        s.b[k] = s.b[k] + prolong_lerp(wy, prolong_lerp(wxb, top[fb], top[sb]),
-                                              prolong_lerp(wxb, bottom[fb], bottom[sb]));
-                }
+                const int f = (k + 1) / 2;
+                s.a[k] = s.a[k] + prolong_lerp(wy[k], xa[f], xa[f + 1]);
+                s.b[k] = s.b[k] + prolong_lerp(wy[k], xb[f], xb[f + 1]);
             }
             // A cell that is no unknown keeps zero: Dirichlet air is read by its liquid
             // neighbours as p = 0; any other such cell has no open face and is never read.
