@@ -492,9 +492,8 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? 4 : 1)
     const Tile t = tiles[blockIdx.x];
     const GridDesc& g = grids[t.grid];
     SolveState& s = *g.state;
-    dependency_wait();
-    if (s.done)
-        return;
+    // The descriptor's fields before the wait: after it they would be one more latency each on the
+    // path (the compiler may not move a load over the wait itself).
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const T* right = static_cast<const T*>(g.lev[0].right);
     const T* down = static_cast<const T*>(g.lev[0].down);
@@ -502,45 +501,32 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? 4 : 1)
     const T* d_old = static_cast<const T*>(g.d[parity]);
     T* d_new = static_cast<T*>(g.d[parity ^ 1]);
     T* q = static_cast<T*>(g.q);
-    const T mz = T(s.mean_z), b = T(s.beta);
-    const int S = g.S;
+    const unsigned char* const air_mask = g.air;
+    const int S = g.S, W = g.W, H = g.H;
     const int gx = t.x0 + 2 * lane;
-    const bool cols = gx < g.W; // the pair's first column lies in the grid
-    const bool in_b = gx + 1 < g.W;
+    const bool cols = gx < W; // the pair's first column lies in the grid
+    const bool in_b = gx + 1 < W;
     // Column just outside the warp: left of the first pair for lane 0, right of the last for 31.
     const int edge_x = lane == 0 ? gx - 1 : gx + 2;
     const bool edge = (lane == 0 && cols) || (lane == 31 && gx + 2 + kPadX < S);
+    // A warp below the grid (a short tile's remainder) has no row above it either.
     P up_w = P{};
-    if (cols)
+    if (cols && t.y0 + ROWS * warp <= H)
         up_w = *reinterpret_cast<const P*>(down + padded_index(S, gx, t.y0 + ROWS * warp - 1));
-    double dot = 0.0;
-#pragma unroll 1
-    for (int pass = 0; pass < ROWS / R; ++pass)
+    // Face weights of two rows, which no kernel of the projection writes: a short tile's only pass has
+    // them on their way before the wait.
+    P w[R], dn[R];
+    T ew[R];
+    auto load_weights = [&](int y0)
     {
-        const int y0 = t.y0 + ROWS * warp + R * pass;
-        P zz[R + 2], dd0[R + 2], w[R], dn[R];
-        T ez[R], ed[R], ew[R];
-#pragma unroll
-        for (int k = 0; k < R + 2; ++k)
-        {
-            const int y = y0 - 1 + k;
-            zz[k] = P{};
-            dd0[k] = P{};
-            if (cols && y >= -1 && y <= g.H)
-            {
-                const long long i = padded_index(S, gx, y);
-                zz[k] = *reinterpret_cast<const P*>(z + i);
-                dd0[k] = *reinterpret_cast<const P*>(d_old + i);
-            }
-        }
 #pragma unroll
         for (int k = 0; k < R; ++k)
         {
             const int y = y0 + k;
             w[k] = P{};
             dn[k] = P{};
-            ez[k] = ed[k] = ew[k] = T(0);
-            if (y < g.H)
+            ew[k] = T(0);
+            if (y < H)
             {
                 const long long i = padded_index(S, gx, y);
                 if (cols)
@@ -549,12 +535,50 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? 4 : 1)
                     dn[k] = *reinterpret_cast<const P*>(down + i);
                 }
                 if (edge)
-                {
-                    const long long e = padded_index(S, edge_x, y);
-                    ez[k] = z[e];
-                    ed[k] = d_old[e];
-                    ew[k] = right[e]; // lane 0: the face between gx - 1 and gx
-                }
+                    ew[k] = right[padded_index(S, edge_x, y)]; // lane 0: the face between gx - 1 and gx
+            }
+        }
+    };
+    constexpr bool kOnePass = ROWS == R;
+    if (kOnePass)
+        load_weights(t.y0 + ROWS * warp);
+    dependency_wait();
+    const double mean_z = s.mean_z, beta = s.beta;
+    if (s.done)
+        return;
+    const T mz = T(mean_z), b = T(beta);
+    double dot = 0.0;
+#pragma unroll 1
+    for (int pass = 0; pass < ROWS / R; ++pass)
+    {
+        const int y0 = t.y0 + ROWS * warp + R * pass;
+        P zz[R + 2], dd0[R + 2];
+        T ez[R], ed[R];
+#pragma unroll
+        for (int k = 0; k < R + 2; ++k)
+        {
+            const int y = y0 - 1 + k;
+            zz[k] = P{};
+            dd0[k] = P{};
+            if (cols && y >= -1 && y <= H)
+            {
+                const long long i = padded_index(S, gx, y);
+                zz[k] = *reinterpret_cast<const P*>(z + i);
+                dd0[k] = *reinterpret_cast<const P*>(d_old + i);
+            }
+        }
+        if (!kOnePass)
+            load_weights(y0);
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+        {
+            const int y = y0 + k;
+            ez[k] = ed[k] = T(0);
+            if (edge && y < H)
+            {
+                const long long e = padded_index(S, edge_x, y);
+                ez[k] = z[e];
+                ed[k] = d_old[e];
             }
         }
         // Directions in the working precision (the operator and the p update read exactly the
@@ -583,17 +607,17 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? 4 : 1)
             if (lane == 31)
                 right_d = edge_dir;
             const P uw = k == 0 ? up_w : dn[k - 1];
-            if (cols && y < g.H)
+            if (cols && y < H)
             {
                 const long long i = padded_index(S, gx, y);
                 const T ca = cur.x, cb = cur.y;
                 T qa = (wl * (ca - left) + w[k].x * (ca - cb)) + (uw.x * (ca - prev.x) + dn[k].x * (ca - next.x));
                 T qb = (w[k].x * (cb - ca) + w[k].y * (cb - right_d)) + (uw.y * (cb - prev.y) + dn[k].y * (cb - next.y));
-                if (g.air)
+                if (air_mask)
                 {
                     // Dirichlet air is no unknown: its direction is zero and its q stays zero,
                     // so its residual stays zero.
-                    const unsigned char* air = g.air + (long long)y * g.W + gx;
+                    const unsigned char* air = air_mask + (long long)y * W + gx;
                     qa = air[0] ? T(0) : qa;
                     qb = in_b && air[1] ? T(0) : qb;
                 }
@@ -668,6 +692,27 @@ __device__ __forceinline__ void add_step(double4& p, double alpha, const typenam
     p.w = step_value(p.w, alpha, double(d.w));
 }
 
+// What a slice's update reads from its grid's descriptor.
+template <typename T> struct UpdateArgs
+{
+    SolveState* state;
+    const T* d;  // this iteration's direction
+    const T* d0; // the other buffer: the pending step's direction in the second of a pair
+    const T* q;
+    T* r;
+    double* p;
+    // Quads of the padded array (S * (H + 2) is a multiple of 8) and per slice; a grid has at most
+    // 2^30 cells, so they and what is formed from them fit 32 bits.
+    int quads, per;
+};
+
+template <typename T> __device__ __forceinline__ UpdateArgs<T> update_args(const GridDesc& g, int parity)
+{
+    const int quads = int((long long)g.S * (g.H + 2) / 4);
+    return {g.state, static_cast<const T*>(g.d[parity ^ 1]), static_cast<const T*>(g.d[parity]), static_cast<const T*>(g.q),
+        static_cast<T*>(g.r), g.p, quads, (quads + g.vec_tiles - 1) / g.vec_tiles};
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads, kUpdateCtasPerSm)
     k_update(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles, int count, int parity)
@@ -677,39 +722,44 @@ __global__ void __launch_bounds__(kVecThreads, kUpdateCtasPerSm)
     // visits the same quads in the same order either way.
     constexpr int U = sizeof(T) == 4 ? 2 : 1;
     allow_dependents();
+    // The first slice's entry and descriptor fields are read before the wait.
+    int i = blockIdx.x;
+    Tile t = i < count ? tiles[i] : Tile{};
+    UpdateArgs<T> a = update_args<T>(grids[t.grid], parity);
     dependency_wait();
     __shared__ double4 total;
     int run = 0; // slices of the current grid finished since the last count
-    for (int i = blockIdx.x; i < count; i += gridDim.x)
+    for (; i < count; i += gridDim.x)
     {
-        const Tile t = tiles[i];
+        if (i != int(blockIdx.x))
+        {
+            t = tiles[i];
+            a = update_args<T>(grids[t.grid], parity);
+        }
         const GridDesc& g = grids[t.grid];
-        SolveState& s = *g.state;
+        SolveState& s = *a.state;
         if (s.done)
             continue;
-        const T* d = static_cast<const T*>(g.d[parity ^ 1]);
-        const T* q = static_cast<const T*>(g.q);
-        T* r = static_cast<T*>(g.r);
+        const T* const d = a.d;
+        const T* const q = a.q;
+        T* const r = a.r;
         const double alpha = s.rz / s.dq;
         // Second of a pair: the first's pending step (its direction is the other buffer).
         const bool update_p = parity == 1;
         const bool pending = update_p && s.p_pending;
         const double alpha0 = s.alpha_pending;
-        const T* d0 = static_cast<const T*>(g.d[parity]);
-        // The padded length S * (H + 2) is a multiple of 8; slices are whole quads.
-        const long long quads = (long long)g.S * (g.H + 2) / 4;
-        const long long per = (quads + g.vec_tiles - 1) / g.vec_tiles;
-        const long long first = per * t.index;
-        const long long last = min(quads, first + per);
+        const T* const d0 = a.d0;
+        const int first = min(a.quads, a.per * t.index);
+        const int last = min(a.quads, first + a.per);
         double sum = 0.0, mx = 0.0, sq = 0.0;
-        for (long long base = first + threadIdx.x; base < last; base += (long long)kVecThreads * U)
+        for (int base = first + int(threadIdx.x); base < last; base += kVecThreads * U)
         {
             Q dv[U], d0v[U], qv[U], rv[U];
             double4 pv[U];
 #pragma unroll
             for (int u = 0; u < U; ++u)
             {
-                const long long j = base + (long long)u * kVecThreads;
+                const int j = base + u * kVecThreads;
                 if (j < last)
                 {
                     qv[u] = reinterpret_cast<const Q*>(q)[j];
@@ -717,7 +767,7 @@ __global__ void __launch_bounds__(kVecThreads, kUpdateCtasPerSm)
                     if (update_p)
                     {
                         dv[u] = reinterpret_cast<const Q*>(d)[j];
-                        pv[u] = reinterpret_cast<const double4*>(g.p)[j];
+                        pv[u] = reinterpret_cast<const double4*>(a.p)[j];
                         if (pending)
                             d0v[u] = reinterpret_cast<const Q*>(d0)[j];
                     }
@@ -726,7 +776,7 @@ __global__ void __launch_bounds__(kVecThreads, kUpdateCtasPerSm)
 #pragma unroll
             for (int u = 0; u < U; ++u)
             {
-                const long long j = base + (long long)u * kVecThreads;
+                const int j = base + u * kVecThreads;
                 if (j >= last)
                     continue;
                 if (update_p)
@@ -735,7 +785,7 @@ __global__ void __launch_bounds__(kVecThreads, kUpdateCtasPerSm)
                     if (pending)
                         add_step<T>(pp, alpha0, d0v[u]);
                     add_step<T>(pp, alpha, dv[u]);
-                    reinterpret_cast<double4*>(g.p)[j] = pp;
+                    reinterpret_cast<double4*>(a.p)[j] = pp;
                 }
                 Q rr;
                 rr.x = T(double(rv[u].x) - alpha * double(qv[u].x));
