@@ -121,10 +121,22 @@ __global__ void k_advect_velocity(const GridDesc* __restrict__ grids, const Tile
     }
 }
 
-// One cell-centred FP64 field (liquid fraction or a component mass) into `next`.
+// Cell-centred FP64 fields (liquid fraction, component masses) into `next`: the back-trace, which is
+// most of the work (two velocity samples, eight loads each, in a serial chain), is done once for up
+// to kAdvectFields of them. (One launch and one trace for each field, and a copy back for each: one
+// tick of 16 uneven grids 6552 -> 6302 us, two Dirichlet steps at 641 x 483 2662 -> 2557 us, a step at
+// 1024 x 1024 8234 -> 8178 us.)
+constexpr int kAdvectFields = 3;
+struct AdvectFields
+{
+    int count;
+    double* field[kAdvectFields];
+    double* next[kAdvectFields];
+};
+
 template <typename T>
 __global__ void k_advect_cells(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles, double s, double half,
-    const double* __restrict__ field, double* __restrict__ next)
+    const AdvectFields f)
 {
     const Tile t = tiles[blockIdx.x];
     const GridDesc& g = grids[t.grid];
@@ -139,8 +151,39 @@ __global__ void k_advect_cells(const GridDesc* __restrict__ grids, const Tile* _
             continue;
         double bx, by;
         trace_back(u, v, W, H, s, half, __dadd_rn(double(i), 0.5), __dadd_rn(double(j), 0.5), bx, by);
-        next[(long long)j * W + i] = sample_clamped(field, W, H, __dsub_rn(bx, 0.5), __dsub_rn(by, 0.5));
+        const double x = __dsub_rn(bx, 0.5), y = __dsub_rn(by, 0.5);
+#pragma unroll
+        for (int n = 0; n < kAdvectFields; ++n)
+            if (n < f.count)
+                f.next[n][(long long)j * W + i] = sample_clamped(f.field[n], W, H, x, y);
     }
+}
+
+// Moves the new values into place: the cell fields, and the velocities with the last of them (null
+// otherwise), all in one launch.
+template <typename T>
+__global__ void k_advect_commit(const AdvectFields f, int cells, const T* __restrict__ u_next, T* __restrict__ u, int faces_u,
+    const T* __restrict__ v_next, T* __restrict__ v, int faces_v)
+{
+    const int stride = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll
+    for (int n = 0; n < kAdvectFields; ++n)
+        if (n < f.count)
+        {
+            const double* __restrict__ from = f.next[n];
+            double* __restrict__ to = f.field[n];
+#pragma unroll 4
+            for (int i = first; i < cells; i += stride)
+                to[i] = from[i];
+        }
+    if (!u)
+        return;
+#pragma unroll 4
+    for (int i = first; i < faces_u; i += stride)
+        u[i] = u_next[i];
+#pragma unroll 4
+    for (int i = first; i < faces_v; i += stride)
+        v[i] = v_next[i];
 }
 
 // FluidGridCPU::sampleVelocity (FluidGridCPU.cpp:465-471) at world positions: positions and

@@ -1818,18 +1818,30 @@ void advect_semi_lagrangian(Grid& g, double dt, bool wait)
     dispatch(g.precision, [&](auto zero)
     {
         using T = decltype(zero);
-        const int fields = 1 + g.components();
-        for (int k = 0; k < fields; ++k)
-        {
-            double* field = k == 0 ? g.fraction : g.masses + size_t(k - 1) * g.cells;
-            FC_LAUNCH(k_advect_cells<T>, p.cells.count, kVecThreads, 0, s, p.d_desc, p.at(p.cells), scale, half, field,
-                g.staging);
-            check(cudaMemcpyAsync(field, g.staging, g.cells * sizeof(double), cudaMemcpyDeviceToDevice, s), "advect");
-        }
+        // The new velocities first: the cell fields trace through the old ones until the commit.
         FC_LAUNCH(k_advect_velocity<T>, p.faces.count, kVecThreads, 0, s, p.d_desc, p.at(p.faces), scale, half,
             static_cast<T*>(g.u_next), static_cast<T*>(g.v_next));
-        check(cudaMemcpyAsync(g.desc.u, g.u_next, g.faces_u * sizeof(T), cudaMemcpyDeviceToDevice, s), "advect");
-        check(cudaMemcpyAsync(g.desc.v, g.v_next, g.faces_v * sizeof(T), cudaMemcpyDeviceToDevice, s), "advect");
+        // Scratch for the new cell fields: the upload staging, and the density and right-hand side,
+        // which every projection (and PLIC transport) forms anew before it reads them.
+        double* const scratch[kAdvectFields] = {g.staging, g.desc.density, g.desc.b};
+        const int fields = 1 + g.components();
+        for (int first = 0; first < fields; first += kAdvectFields)
+        {
+            AdvectFields f{};
+            f.count = std::min(kAdvectFields, fields - first);
+            for (int n = 0; n < f.count; ++n)
+            {
+                const int k = first + n;
+                f.field[n] = k == 0 ? g.fraction : g.masses + size_t(k - 1) * g.cells;
+                f.next[n] = scratch[n];
+            }
+            const bool last = first + f.count == fields;
+            FC_LAUNCH(k_advect_cells<T>, p.cells.count, kVecThreads, 0, s, p.d_desc, p.at(p.cells), scale, half, f);
+            // Four elements of the largest array a thread.
+            FC_LAUNCH(k_advect_commit<T>, blocks_for((std::max(g.faces_u, g.faces_v) + 3) / 4), 256, 0, s, f, int(g.cells),
+                static_cast<const T*>(g.u_next), last ? static_cast<T*>(g.desc.u) : nullptr, int(g.faces_u),
+                static_cast<const T*>(g.v_next), last ? static_cast<T*>(g.desc.v) : nullptr, int(g.faces_v));
+        }
     });
     if (wait)
         check(cudaStreamSynchronize(s), "advect");
