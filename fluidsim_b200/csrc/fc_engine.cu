@@ -848,9 +848,10 @@ __global__ void __launch_bounds__(kVecThreads) k_count_open(const GridDesc* __re
 __global__ void k_loop_condition(const GridDesc* grids, int n, int* body_count, int cap, cudaGraphConditionalHandle handle)
 {
     allow_dependents();
+    const SolveState* const first = int(threadIdx.x) < n ? grids[threadIdx.x].state : nullptr;
     dependency_wait();
-    int running = 0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
+    int running = first && first->done == 0;
+    for (int i = threadIdx.x + blockDim.x; i < n; i += blockDim.x)
         running |= grids[i].state->done == 0;
     running = __syncthreads_or(running);
     if (threadIdx.x == 0)
