@@ -2130,7 +2130,7 @@ template <typename T> void viscosity_cycle(ViscWork& w, size_t l, void* b, doubl
         return;
     }
     const int blocks = ceil_div((L.w + 1) * (L.h + 1), kViscThreads);
-    auto tiles = [](const ViscLevel& v) { return dim3(ceil_div(v.w + 1, kViscTileX), ceil_div(v.h + 1, kViscTileY)); };
+    auto tiles = [](const ViscLevel& v) { return ceil_div(v.w + 1, kViscTileX) * ceil_div(v.h + 1, kViscTileY); };
     auto smooth = [&]
     {
         FC_LAUNCH_DEP(k_visc_smooth<T>, blocks, kViscThreads, 0, s, L, dt, b, w.state);

@@ -510,6 +510,15 @@ __device__ __forceinline__ double transfer_weight(int f, bool half, int p, int l
 constexpr int kViscTileX = 32, kViscTileY = 8;
 constexpr int kViscFineX = 2 * kViscTileX + 2, kViscFineY = 2 * kViscTileY + 2;
 
+// Origin of a block's tile in a lattice of w + 1 columns. The tiles are counted in one grid dimension:
+// a tall thin lattice has more rows of them than a second one holds.
+__device__ __forceinline__ void visc_tile(int w, int& x0, int& y0)
+{
+    const int columns = w / kViscTileX + 1; // ceil((w + 1) / kViscTileX)
+    x0 = int(blockIdx.x % columns) * kViscTileX;
+    y0 = int(blockIdx.x / columns) * kViscTileY;
+}
+
 // The coarse right-hand side at node (px, py): the transpose of the prolongation applied to the 4 x 4
 // fine residuals 2p - 1 .. 2p + 2, q(row, column), summed in the stencil's row order.
 template <typename T, typename Q>
@@ -581,7 +590,8 @@ __global__ void __launch_bounds__(kViscThreads) k_visc_restrict(ViscLevel fine, 
     __shared__ T2 res[kViscFineY][kViscFineX];
     if (visc_stopped(state))
         return;
-    const int X0 = blockIdx.x * kViscTileX, Y0 = blockIdx.y * kViscTileY;
+    int X0, Y0;
+    visc_tile(coarse.w, X0, Y0);
     for (int i = threadIdx.x; i < kViscFineX * kViscFineY; i += kViscThreads)
     {
         const int j = i / kViscFineX, k = i - j * kViscFineX;
@@ -657,7 +667,8 @@ __global__ void __launch_bounds__(kViscThreads) k_visc_prolong_smooth(ViscLevel 
     __shared__ T2 tile[RY * RX];
     if (visc_stopped(state))
         return;
-    const int X0 = blockIdx.x * kViscTileX, Y0 = blockIdx.y * kViscTileY;
+    int X0, Y0;
+    visc_tile(fine.w, X0, Y0);
     for (int i = threadIdx.x; i < RX * RY; i += kViscThreads)
     {
         // Clamped like the operator's reads: the ring beyond the lattice repeats its edge.

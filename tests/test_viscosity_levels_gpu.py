@@ -39,3 +39,29 @@ def test_solve_matches_restatement(oracle, size, precision, bound):
     if precision == "fp64":
         assert it == expected_it
     assert np.abs(s.u - eu).max() <= bound * scale and np.abs(s.v - ev).max() <= bound * scale
+
+
+def test_tall_thin_lattice_equals_its_transpose():
+    """More rows of tiles than a launch's second dimension holds (65,535): the solve runs, and equals
+    the transposed one to the stop rule's tolerance."""
+    w, h, dt = 2, 530000, 1.0 / 120.0
+    dx = 1.0 / 512.0
+    y = np.arange(h)
+    rng = np.random.default_rng(5)
+    share = np.repeat((0.5 + 0.5 * np.sin(0.003 * y))[:, None], w, axis=1)
+    u, v = np.zeros((h, w + 1)), np.zeros((h + 1, w))
+    u[:, 1] = rng.uniform(-1, 1, h)
+    v[1:-1] = rng.uniform(-1, 1, (h - 1, w))
+    out = []
+    for transpose in (False, True):
+        f = share.T if transpose else share
+        g = FluidGrid(*((h, w) if transpose else (w, h)), dx, "fp64")
+        g.configureMaterials([900.0], [40.0], [2.0], [0.01])
+        g.upload(FluidGridState(f, v.T if transpose else u, u.T if transpose else v, None, [900.0 * f * dx * dx],
+                                [40.0 * (1.0 - f) * dx * dx]))
+        it, residual = g.applyViscosity(dt, 1e-4)
+        assert it > 0 and residual <= 1.1e-4
+        s = g.download()
+        out.append((s.v.T, s.u.T) if transpose else (s.u, s.v))
+    for a, b in zip(*out):
+        assert np.abs(a - b).max() <= 1e-8 * max(np.abs(b).max(), 1e-30)
