@@ -422,6 +422,9 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
     dependency_wait();
     const int done = state.done;
     const double mean_r = first == 0 ? state.mean_r : 0.0;
+    // Only the fine level's right-hand side has a mean to take off: a coarser one is restricted from
+    // a residual that has none of it left.
+    const double level_mean = role == 0 ? mean_r : 0.0;
     if (role == 0)
     {
 #pragma unroll
@@ -508,9 +511,8 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
 #pragma unroll
             for (int k = 0; k < kTailK; ++k)
             {
-                // Only the fine level's right-hand side has a mean to take off (else mean_r is zero).
-                s.ra[k] = s.ia[k] > T(0) ? minus_mean(s.ra[k], mean_r) : T(0);
-                s.rb[k] = s.ib[k] > T(0) ? minus_mean(s.rb[k], mean_r) : T(0);
+                s.ra[k] = s.ia[k] > T(0) ? minus_mean(s.ra[k], level_mean) : T(0);
+                s.rb[k] = s.ib[k] > T(0) ? minus_mean(s.rb[k], level_mean) : T(0);
                 s.a[k] = s.b[k] = T(0);
             }
         }

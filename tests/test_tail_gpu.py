@@ -82,3 +82,30 @@ def test_fp32_tail_stays_close_to_fp64(size):
         out[precision] = g.applyPreconditioner(residual)
     scale = max(1.0, np.abs(out["fp64"]).max())
     assert np.abs(out["fp32"] - out["fp64"]).max() <= 5e-4 * scale
+
+
+# Grids whose fine level and at least one more smoothed level are in the tail: at the default
+# threshold, and at the largest one.
+WHOLE = [(20, 20, 1024), (32, 32, 1024), (64, 16, 1024), (33, 31, 1024), (50, 41, 4096), (64, 64, 4096)]
+
+
+@pytest.mark.parametrize("precision,bound", [("fp64", 1e-10), ("fp32", 5e-4), ("mixed", 5e-4)])
+@pytest.mark.parametrize("w,h,cells", WHOLE)
+def test_residual_mean_is_taken_off_the_fine_level_alone(oracle, w, h, cells, precision, bound):
+    """The preconditioner acts on residual - residual_mean (FluidGridCPU.cpp:1712-1726): a constant
+    residual gives exact zeros, and a shifted one what the unshifted one gives. The residual is a
+    multiple of 2^-16, so the shifted one is exact in FP32 too and the bounds are those above."""
+    density, residual = _case(w, h)
+    residual = np.round(residual * 65536.0) / 65536.0
+    inv_u, inv_v, _ = oracle.coefficients(density)
+    mg = oracle.Multigrid(w, h)
+    assert mg.rebuild(inv_u, inv_v)
+    expected = mg.apply(residual)
+    s = scenes.Scene(w, h, 1.0, 1.0, 1.0, 1.0, np.ones((h, w)), np.zeros((h, w + 1)), np.zeros((h + 1, w)),
+                     liquid_mass=[density], gas_mass=[np.zeros((h, w))])
+    g = FluidGrid(w, h, 1.0, precision)
+    scenes.upload_scene(g, s)
+    g.setTailCells(cells)
+    assert np.all(g.applyPreconditioner(np.full((h, w), 7.0), 7.0) == 0.0)
+    z = g.applyPreconditioner(residual + 3.5, 3.5)
+    assert np.abs(z - expected).max() <= bound * max(1.0, np.abs(expected).max())
