@@ -1050,6 +1050,9 @@ struct Plan
     int cells_max[kMaxLevels] = {}; // most cells of any grid's level, per level
     size_t tail_smem = 0;
     int tail_threads = 0;
+    // First tail level of each grid when the plan was made: the tiles and the tail's launch follow
+    // from it, so a plan is remade once a grid's tail moves (plan_current).
+    std::vector<int> tails;
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;
     int graph_cap = -1;
@@ -1179,6 +1182,7 @@ std::unique_ptr<Plan> make_plan(const std::vector<Grid*>& grids, cudaStream_t st
         plan->max_tail = std::max(plan->max_tail, g->tail);
         plan->tail_smem = std::max(plan->tail_smem, g->tail_smem);
         plan->tail_threads = std::max(plan->tail_threads, g->tail_threads);
+        plan->tails.push_back(g->tail);
         for (size_t l = 0; l < g->levels.size(); ++l)
             plan->cells_max[l] = std::max(plan->cells_max[l], g->levels[l].w * g->levels[l].h);
     }
@@ -1245,6 +1249,15 @@ std::unique_ptr<Plan> make_plan(const std::vector<Grid*>& grids, cudaStream_t st
     plan->h_states = new SolveState[n]();
     upload_descriptors(*plan);
     return plan;
+}
+
+// Whether the grids' tails still start where they did when the plan was made.
+bool plan_current(const Plan& p)
+{
+    for (int i = 0; i < p.n(); ++i)
+        if (p.grids[i]->tail != p.tails[i])
+            return false;
+    return true;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -2497,8 +2510,8 @@ double time_kernel(Grid& g, int kernel, int repeats)
 // the same red-black sweeps, transfers and coarsest solve. The tuner times V-cycles of a plan
 // under each candidate and keeps the fastest.
 
-// Applies a tail threshold to a grid. The grid's single-grid plan is rebuilt on next use; the
-// caller rebuilds any batch plan holding it.
+// Applies a tail threshold to a grid. The grid's single-grid plan is rebuilt on next use, and so is
+// a batch plan that holds it (fc_batch_project).
 void set_tail_cells(Grid& g, int cells)
 {
     g.tail_cells = cells;
@@ -3956,8 +3969,16 @@ int fc_batch_project(fc_batch* batch, const double* dts, int max_iterations, dou
         for (size_t i = 0; i < batch->grids.size(); ++i)
             if (!(dts[i] > 0.0))
                 fail(FC_ERR_INVALID_ARGUMENT, "time steps must be positive");
+        // Grids may have changed (obstacles, materials, tail threshold) since the batch was made. With
+        // a moved tail the plan is made again, on its stream, which the caller may hold.
+        if (!fc::plan_current(*batch->plan))
+        {
+            fc::Plan& old = *batch->plan;
+            auto made = fc::make_plan(old.grids, old.stream);
+            std::swap(made->own_stream, old.own_stream);
+            batch->plan = std::move(made);
+        }
         fc::Plan& p = *batch->plan;
-        // Grids may have changed (obstacles, materials) since the batch was made.
         for (Grid* g : p.grids)
         {
             g->desc.solid = g->has_solid ? g->solid : nullptr;

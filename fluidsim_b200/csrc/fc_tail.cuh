@@ -331,23 +331,14 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
     // plain loads for the set-up, and with the tables and the coarsest inverse by bulk copy for the
     // cycle.
     const int smoothed = table->smoothed, first = table->first, tables = table->tables, zeroed = table->zeroed;
-    // Bulk copies write 16-byte aligned shared addresses only: a misplaced buffer is reported.
-    const bool aligned = (smem_address(tail_smem) & 15u) == 0;
-    if (threadIdx.x == 0 && aligned)
-    {
-        mbarrier_init(&bar, 1);
-        fence_async_shared();
-        const unsigned bytes = kTailHeader + unsigned(tables) * sizeof(T);
-        mbarrier_expect_tx(&bar, bytes + unsigned(kTailInverseBytes));
-        bulk_load(tail_smem + kTailSolveBytes, table, bytes, &bar);
-        bulk_load(inverse, g.coarse_inverse, unsigned(kTailInverseBytes), &bar);
-    }
+    const int elements = table->elements;
     // This warp's level (-1: none).
-    int role = -1, level_warp = warp;
+    int role = -1, level_warp = warp, warps_needed = 0;
 #pragma unroll
     for (int i = 0; i < kTailMaxSmoothed; ++i)
     {
         const int warps = table->place[i].warps; // zero where there is no such level
+        warps_needed += warps;
         if (role < 0)
         {
             if (level_warp < warps)
@@ -355,6 +346,19 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
             else
                 level_warp -= warps;
         }
+    }
+    // Bulk copies write 16-byte aligned shared addresses only, and a level's barrier waits for all its
+    // warps: a misplaced buffer or a table that this launch is too small for is reported.
+    const bool ready = (smem_address(tail_smem) & 15u) == 0 && 32 * warps_needed <= kThreads &&
+        unsigned(kTailSolveBytes) + kTailHeader + unsigned(elements) * sizeof(T) <= dynamic_smem_bytes();
+    if (threadIdx.x == 0 && ready)
+    {
+        mbarrier_init(&bar, 1);
+        fence_async_shared();
+        const unsigned bytes = kTailHeader + unsigned(tables) * sizeof(T);
+        mbarrier_expect_tx(&bar, bytes + unsigned(kTailInverseBytes));
+        bulk_load(tail_smem + kTailSolveBytes, table, bytes, &bar);
+        bulk_load(inverse, g.coarse_inverse, unsigned(kTailInverseBytes), &bar);
     }
     const TailPlace& place = table->place[max(role, 0)];
     const int S = place.S;
@@ -403,12 +407,15 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
     const T* const rhs = static_cast<const T*>(table->rhs);
     T* const out = static_cast<T*>(table->out);
     // Edges and lines start at zero: what lies outside a level is never written.
-    for (int i = threadIdx.x; i < zeroed; i += blockDim.x)
-        m[tables + i] = T(0);
-    if (threadIdx.x < kMaxCoarse)
-        coarse_rhs[threadIdx.x] = 0.0;
+    if (ready)
+    {
+        for (int i = threadIdx.x; i < zeroed; i += blockDim.x)
+            m[tables + i] = T(0);
+        if (threadIdx.x < kMaxCoarse)
+            coarse_rhs[threadIdx.x] = 0.0;
+    }
     __syncthreads();
-    if (stage_failed(aligned && mbarrier_wait(&bar, 0), g.state))
+    if (stage_failed(ready && mbarrier_wait(&bar, 0), g.state))
         return;
     const TailPlace& own = shared_table.place[max(role, 0)];
     const TailPlace& finer = shared_table.place[max(role - 1, 0)];

@@ -1,5 +1,5 @@
-"""Autotuning of the multigrid schedule: the tail threshold changes which kernels run (one-block
-shared-memory tail or strip kernels), not the method, so every threshold must give the same
+"""Autotuning of the multigrid schedule: the tail threshold changes which kernels run (one-CTA
+tail or strip kernels), not the method, so every threshold must give the same
 projection to rounding."""
 import numpy as np
 import pytest
@@ -60,4 +60,34 @@ def test_batch_autotune_then_batch_equals_single():
         assert rs.iterations == r.iterations
         a, c = single.download(), g.download()
         assert np.array_equal(a.u, c.u) and np.array_equal(a.pressure, c.pressure)
+    b.destroy()
+
+
+@pytest.mark.parametrize("before,after", [(256, 4096), (4096, 64), (64, 1024)])
+def test_batch_follows_its_members_tail_thresholds(before, after):
+    """A member's threshold moves after the batch was made, which changes its levels above the tail,
+    the tail's shared memory and its warps (64 x 50: one warp at 256 cells, eighteen at 4096): the
+    batch still computes what each grid computes alone, and keeps its stream."""
+    batch_scenes = [scenes.random_pool(w, h, seed=w + h, fill=0.6, cell_size=1.0 / w)
+                    for w, h in [(64, 50), (190, 130), (20, 20)]]
+    grids = [_grid(s, "fp32") for s in batch_scenes]
+    for g in grids:
+        g.setTailCells(before)
+    b = ProjectionBatch(grids)
+    dts = [s.dt for s in batch_scenes]
+    stream = b.stream()
+    assert all(r.solve_status == "converged" for r in b.project(dts, 300, 1e-6, relative_tolerance=1e-6))
+    for changed in (grids[:1], grids):
+        for g in changed:
+            g.setTailCells(after)
+        for g, s in zip(grids, batch_scenes):
+            scenes.upload_scene(g, s)
+        results = b.project(dts, 300, 1e-6, relative_tolerance=1e-6)
+        assert b.stream() == stream
+        for s, g, r in zip(batch_scenes, grids, results):
+            single = _grid(s, "fp32")
+            single.setTailCells(after if g in changed else before)
+            assert single.project(s.dt, 300, 1e-6, relative_tolerance=1e-6).iterations == r.iterations
+            x, y = single.download(), g.download()
+            assert np.array_equal(x.u, y.u) and np.array_equal(x.pressure, y.pressure)
     b.destroy()
