@@ -13,7 +13,7 @@
 //  * The restriction's sums along x come from the residual registers; the coarse level's lanes
 //    sum them along y straight into their right-hand side registers.
 //  * The coarsest solve is one matrix product: its mean removals are folded into the inverse when
-//    it is built (k_rebuild_tail).
+//    it is built (k_rebuild_tail), unless obstacles seal off a part of the level.
 //  * The layout and the transfer weights come in one host-built block (TailTable).
 //
 // Measured with fc_time_kernel on a 512 x 512 grid (levels 32 x 32, 16 x 16, 8 x 8), before this
@@ -129,9 +129,19 @@ inline void tail_layout(TailTable& t, int plane)
 
 // The coarsest inverse's rows are 72 doubles apart, in global and in shared memory: the four rows
 // that a warp reads then cover every bank twice. It is copied whole; rows and columns beyond the
-// level's cells are zero.
+// level's cells are zero. One more row and column serve an inverse without folded means (TailMeans).
 constexpr int kTailInverseStride = 72;
-constexpr size_t kTailInverseBytes = size_t(kMaxCoarse) * kTailInverseStride * sizeof(double);
+constexpr size_t kTailInverseBytes = size_t(kMaxCoarse + 1) * kTailInverseStride * sizeof(double);
+
+// Elements of the inverse that say how the solve takes its means: the column sums (row kMaxCoarse),
+// one for each open cell and zero for another (column kMaxCoarse), and the share of a cell in a
+// mean, zero where the solve takes none (folded, or Dirichlet air).
+struct TailMeans
+{
+    static __host__ __device__ constexpr int sums(int cell) { return kMaxCoarse * kTailInverseStride + cell; }
+    static __host__ __device__ constexpr int open(int cell) { return cell * kTailInverseStride + kMaxCoarse; }
+    static constexpr int share = kMaxCoarse * kTailInverseStride + kMaxCoarse;
+};
 
 // Dynamic shared memory: the coarsest inverse, its right-hand side in FP64, the table's header, and
 // the levels' elements (at most 10840 in FP32 and 5912 in FP64 over every level shape a tail
@@ -323,7 +333,7 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
     const TailTable* const table = static_cast<const TailTable*>(g.tail_table);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double* const inverse = reinterpret_cast<double*>(tail_smem);
-    double* const coarse_rhs = inverse + kMaxCoarse * kTailInverseStride;
+    double* const coarse_rhs = inverse + kTailInverseBytes / sizeof(double);
     const TailTable& shared_table = *reinterpret_cast<const TailTable*>(tail_smem + kTailSolveBytes);
     T* const m = tail_elements<T>();
     __shared__ uint64_t bar;
@@ -446,44 +456,64 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
     if (done)
         return;
 
-    // The coarsest level (at most 64 cells): mean-free, explicit inverse, mean-zero gauge in one
-    // product (PressureMultigrid.cpp:347-384), its solution to last.sol. Eight threads per row, each
-    // with every eighth entry in two chains.
+    // The coarsest level (at most 64 cells): mean-free, explicit inverse, mean-zero gauge
+    // (PressureMultigrid.cpp:347-384), its solution to last.sol. Eight threads per row, each with every
+    // eighth entry in two chains. With the means folded into the inverse that is one product; otherwise
+    // the right-hand side's mean comes off first (and is returned), and the solution's from the row of
+    // the column sums.
     auto solve_coarsest = [&](T value)
     {
-        if (int(threadIdx.x) < cells)
-            coarse_rhs[threadIdx.x] = double(value);
-        __syncthreads();
+        const double share = inverse[TailMeans::share];
+        const bool means = share != 0.0;
         const int part = threadIdx.x & 7;
-#pragma unroll
-        for (int base = 0; base < kMaxCoarse; base += kThreads / 8)
+        double mean = 0.0, gauge = 0.0;
+        auto product = [&](const double* row)
         {
-            const int row = base + int(threadIdx.x >> 3);
+            const double* a = row + part;
             double z = 0.0, z1 = 0.0;
-            if (row < kMaxCoarse)
-            {
-                const double* a = inverse + row * kTailInverseStride + part;
 #pragma unroll
-                for (int i = 0; i < kMaxCoarse / 16; ++i)
-                {
-                    z += a[16 * i] * coarse_rhs[part + 16 * i];
-                    z1 += a[16 * i + 8] * coarse_rhs[part + 16 * i + 8];
-                }
+            for (int i = 0; i < kMaxCoarse / 16; ++i)
+            {
+                z += a[16 * i] * coarse_rhs[part + 16 * i];
+                z1 += a[16 * i + 8] * coarse_rhs[part + 16 * i + 8];
             }
             z += z1;
             z += __shfl_xor_sync(0xffffffffu, z, 1);
             z += __shfl_xor_sync(0xffffffffu, z, 2);
             z += __shfl_xor_sync(0xffffffffu, z, 4);
+            return z;
+        };
+        if (int(threadIdx.x) < cells)
+            coarse_rhs[threadIdx.x] = double(value);
+        __syncthreads();
+        if (means)
+        {
+            for (int i = lane; i < cells; i += 32)
+                mean += inverse[TailMeans::open(i)] * coarse_rhs[i];
+            mean = warp_sum(mean) * share;
+            __syncthreads();
+            if (int(threadIdx.x) < cells)
+                coarse_rhs[threadIdx.x] -= mean;
+            __syncthreads();
+            gauge = product(inverse + TailMeans::sums(0)) * share;
+        }
+#pragma unroll
+        for (int base = 0; base < kMaxCoarse; base += kThreads / 8)
+        {
+            const int row = base + int(threadIdx.x >> 3);
+            const double z = product(inverse + min(row, kMaxCoarse - 1) * kTailInverseStride);
             if (row < cells && part == 0)
-                m[last.sol + row] = T(z);
+                m[last.sol + row] = means && inverse[TailMeans::open(row)] == 0.0 ? T(0) : T(z - gauge);
         }
         __syncthreads();
+        return mean;
     };
     if (smoothed == 0)
     {
         // A level of at most 64 cells is all the tail has: its right-hand side as it stands (less the
         // residual's mean on the fine level; closed cells have zero columns), and straight out.
-        solve_coarsest(int(threadIdx.x) < cells ? minus_mean(rhs[padded_index32(S, cx, cy)], mean_r) : T(0));
+        const double mean =
+            mean_r + solve_coarsest(int(threadIdx.x) < cells ? minus_mean(rhs[padded_index32(S, cx, cy)], mean_r) : T(0));
         if (int(threadIdx.x) < cells)
             out[padded_index32(S, cx, cy)] = m[last.sol + threadIdx.x];
         if (first == 0 && threadIdx.x == 0)
@@ -495,8 +525,8 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
                 sz += z;
                 srz += coarse_rhs[i] * z;
             }
-            // coarse_rhs holds r - mean r: sum r z = sum (r - mean r) z + mean r sum z.
-            finish_preconditioner(state, sz, srz + mean_r * sz);
+            // coarse_rhs holds r - mean: sum r z = sum (r - mean) z + mean sum z.
+            finish_preconditioner(state, sz, srz + mean * sz);
         }
         return;
     }
@@ -638,21 +668,137 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
 //
 // Dense pinned operator of the coarsest level and its inverse in FP64; one CTA per grid
 // (PressureMultigrid.cpp:300-345, factorCoarsest). The first open cell is pinned (the reference
-// pins cell 0; with no obstacle the two are the same), Dirichlet air pins none. Gauss-Jordan
-// elimination without pivoting: on a symmetric positive matrix its pivots are the squares of the
-// Cholesky factor's diagonal, so a non-positive or non-finite one marks the same breakdown
-// (PressureMultigrid.cpp:334-335). Rows and columns of cells that are no unknown are kept as
-// those of the identity during the elimination and written as zeros.
+// pins cell 0; with no obstacle the two are the same), Dirichlet air pins none. A non-positive or
+// non-finite pivot of the Cholesky factor marks the breakdown (:334-335). Rows and columns of cells
+// that are no unknown are kept as those of the identity during the elimination and written as zeros.
 //
-// The solve removes the mean of its right-hand side and gives its solution a mean-zero gauge
-// (:347-384); both are linear, so the stored matrix is C inverse C with C = I - 1 1^T / open over
-// the open cells (the pinned one included), and the tail applies one matrix.
+// Gauss-Jordan elimination without pivoting: its pivots are the squares of the factor's diagonal, to
+// rounding. A step publishes the pivot row and column in shared memory, double-buffered, so it costs
+// one barrier and one division deep. The solve removes the mean of its right-hand side and gives
+// its solution a mean-zero gauge (:347-384); both are linear, so the stored matrix is C inverse C
+// with C = I - 1 1^T / open over the open cells (the pinned one included).
 //
-// Eight threads hold a row in registers (every eighth column); a step publishes the pivot row and
-// column in shared memory, double-buffered, so it costs one barrier and one division deep.
-constexpr int kCoarseThreads = 8 * kMaxCoarse;
+// Where obstacles seal off a part of the level the operator is singular: that part's last pivot is
+// a rounding error, whose sign decides between breakdown and solve, and the inverse has entries of
+// 1e16, in which folded means would drown every other part's. So if a pivot is not above kSealedPivot
+// of the largest diagonal, the factor is formed again by the reference's column loop (invert_factor)
+// and the means are left to the solve. (Gauss-Jordan pivots decided 26 of 96 sealed 8 x 8 scenes
+// differently from the column loop.) Rounding moves either method's pivots by at most a few times
+// 64 epsilon of the largest diagonal (the Schur complements of this diagonally dominant matrix do not
+// grow), so above the limit both accept. Densities of 1000 : 1 leave pivots of 1e-5 and more.
+// The whole kernel on a 64 x 64 grid in FP32: 41 us, 98 us where a wall across it needs the column loop.
+constexpr double kSealedPivot = 1.0 / (1 << 24);
 
-template <typename T> __global__ void __launch_bounds__(kCoarseThreads) k_rebuild_tail(const GridDesc* __restrict__ grids)
+// Eight threads hold a row in registers (every eighth column).
+constexpr int kCoarseThreads = 8 * kMaxCoarse;
+constexpr int kCoarseColumns = kMaxCoarse / 8;
+struct CoarseRow
+{
+    double a[kCoarseColumns]; // columns part, part + 8, ...
+    int r, part;
+};
+
+// The inverse of the operator in `row` by its Cholesky factor, in the place of the operator; true
+// if a pivot is not positive or not finite. `unknowns` has the bits of the unknowns' cells.
+//
+// The factor L is formed right-looking: every entry takes the reference's subtractions in the
+// reference's order (PressureMultigrid.cpp:313-339), each product fused into its subtraction. Y = L^-1
+// takes the place of the columns L is done with, and the inverse is Y^T Y. Step k publishes one
+// vector: column k of L below the diagonal, and row k of Y up to it. Every warp carries the diagonal,
+// two entries a lane, so its next pivot needs no other warp: one barrier a step, double-buffered.
+static __device__ __noinline__ bool invert_factor(CoarseRow& row, const double* diagonal, unsigned long long unknowns, int cells)
+{
+    constexpr int N = kMaxCoarse, E = kCoarseColumns;
+    __shared__ double factor[N * kTailInverseStride];
+    __shared__ double step[2][N];
+    __shared__ int failed;
+    const int r = row.r, part = row.part, lane = threadIdx.x & 31;
+    const int first_row = r & ~3, last_row = first_row + 3; // of the warp
+    double a[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+        a[i] = row.a[i];
+    double d0 = diagonal[lane], d1 = diagonal[lane + 32];
+    int buf = 0;
+    if (threadIdx.x == 0)
+        failed = 0;
+    __syncthreads();
+#pragma unroll 1
+    for (unsigned long long rest = unknowns; rest != 0; rest &= rest - 1, buf ^= 1)
+    {
+        const int k = __ffsll((long long)rest) - 1;
+        if (last_row >= k)
+        {
+            const double value = __shfl_sync(0xffffffffu, k < 32 ? d0 : d1, k & 31);
+            const double pivot = sqrt(value);
+            double own = a[0];
+#pragma unroll
+            for (int i = 1; i < E; ++i)
+                own = i == k >> 3 ? a[i] : own;
+            // Row k's threads divide one, the others (those of column k count) their entry; a zero
+            // stays zero without a division, which would take its slow path.
+            const bool zero = own == 0.0;
+            const double quotient = (r == k || zero ? 1.0 : own) / pivot;
+            if (r == k)
+            {
+                if (!(value > 0.0) || !isfinite(value))
+                    failed = 1;
+#pragma unroll
+                for (int i = 0; i < E; ++i)
+                {
+                    const int c = part + 8 * i;
+                    if (c <= k)
+                        step[buf][c] = a[i] = c == k ? quotient : a[i] * quotient;
+                }
+            }
+            else if (r > k && part == (k & 7))
+                step[buf][r] = zero ? 0.0 : quotient;
+        }
+        __syncthreads();
+        if (last_row > k)
+        {
+            const double l0 = step[buf][lane], l1 = step[buf][lane + 32];
+            if (lane > k)
+                d0 = fma(-l0, l0, d0);
+            if (lane + 32 > k)
+                d1 = fma(-l1, l1, d1);
+            if (r > k)
+            {
+                const double lr = step[buf][r];
+#pragma unroll
+                for (int i = 0; i < E; ++i)
+                {
+                    const int c = part + 8 * i;
+                    a[i] = fma(-lr, step[buf][c], c == k ? 0.0 : a[i]);
+                }
+            }
+        }
+    }
+    const bool mine = unknowns >> r & 1;
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+    {
+        const int c = part + 8 * i;
+        factor[r * kTailInverseStride + c] = mine && c <= r && (unknowns >> c & 1) ? a[i] : 0.0;
+        a[i] = 0.0;
+    }
+    __syncthreads();
+    // Entry (r, c) sums Y[k][r] Y[k][c] over k >= max(r, c): the terms before it are zero.
+    for (int k = first_row; k < cells; ++k)
+    {
+        const double* const y = factor + k * kTailInverseStride;
+        const double yr = y[r];
+#pragma unroll
+        for (int i = 0; i < E; ++i)
+            a[i] = fma(yr, y[part + 8 * i], a[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+        row.a[i] = a[i];
+    return failed != 0;
+}
+
+template <typename T> __global__ void __launch_bounds__(kCoarseThreads, 1) k_rebuild_tail(const GridDesc* __restrict__ grids)
 {
     dependent_start();
     const GridDesc& g = grids[blockIdx.x];
@@ -666,15 +812,14 @@ template <typename T> __global__ void __launch_bounds__(kCoarseThreads) k_rebuil
     }
     const LevelDesc& l = g.lev[level];
     const int cells = l.w * l.h;
-    constexpr int N = kMaxCoarse, E = kMaxCoarse / 8;
-    __shared__ double pivot_row[2][N], pivot_col[2][N], row_mean[N];
+    constexpr int N = kMaxCoarse, E = kCoarseColumns;
+    __shared__ double pivot_row[2][N], pivot_col[2][N], row_mean[N], diagonal[N];
     __shared__ unsigned char open[N];
-    __shared__ int pinned_shared, open_shared, failed;
-    __shared__ double mean_shared;
+    __shared__ int sealed;
     const T* right = static_cast<const T*>(l.right);
     const T* down = static_cast<const T*>(l.down);
     const bool dirichlet = g.air != nullptr;
-    const int r = threadIdx.x >> 3, part = threadIdx.x & 7;
+    const int r = threadIdx.x >> 3, part = threadIdx.x & 7, lane = threadIdx.x & 31;
     const int x = r % l.w, y = r / l.w;
     double diag = 0.0, wl = 0.0, wr = 0.0, wu = 0.0, wd = 0.0;
     if (r < cells)
@@ -687,44 +832,45 @@ template <typename T> __global__ void __launch_bounds__(kCoarseThreads) k_rebuil
         diag = ((wl + wr) + wu) + wd;
     }
     if (part == 0)
+    {
         open[r] = r < cells && diag > 0.0 && !(dirichlet && held_cell<T>(g, level, x, y)) ? 1 : 0;
+        diagonal[r] = diag;
+    }
     if (threadIdx.x == 0)
-        failed = 0;
+        sealed = 0;
     __syncthreads();
-    if (threadIdx.x < 32)
-    {
-        const unsigned lo = __ballot_sync(0xffffffffu, open[threadIdx.x] != 0);
-        const unsigned hi = __ballot_sync(0xffffffffu, open[threadIdx.x + 32] != 0);
-        if (threadIdx.x == 0)
-        {
-            const unsigned long long mask = (static_cast<unsigned long long>(hi) << 32) | lo;
-            open_shared = __popcll(mask);
-            pinned_shared = dirichlet || !mask ? -1 : __ffsll((long long)mask) - 1;
-        }
-    }
-    __syncthreads();
-    const int pinned = pinned_shared, open_cells = open_shared;
-    auto unknown = [&](int c) { return open[c] != 0 && c != pinned; };
+    const unsigned low = __ballot_sync(0xffffffffu, open[lane] != 0);
+    const unsigned high = __ballot_sync(0xffffffffu, open[lane + 32] != 0);
+    const unsigned long long open_mask = (static_cast<unsigned long long>(high) << 32) | low;
+    const unsigned long long unknowns = dirichlet ? open_mask : open_mask & (open_mask - 1); // less the first open cell
+    auto unknown = [&](int c) { return (unknowns >> c & 1) != 0; };
     const bool mine = unknown(r);
+    double largest = fmax(diagonal[lane], diagonal[lane + 32]);
+    for (int offset = 16; offset > 0; offset >>= 1)
+        largest = fmax(largest, __shfl_xor_sync(0xffffffffu, largest, offset));
     double a[E];
-#pragma unroll
-    for (int i = 0; i < E; ++i)
+    auto form = [&]
     {
-        const int c = part + 8 * i;
-        double value = c == r ? (mine ? diag : 1.0) : 0.0;
-        if (mine && c != r && unknown(c))
+#pragma unroll
+        for (int i = 0; i < E; ++i)
         {
-            if (x > 0 && c == r - 1)
-                value = -wl;
-            if (x + 1 < l.w && c == r + 1)
-                value = -wr;
-            if (c == r - l.w)
-                value = -wu;
-            if (c == r + l.w)
-                value = -wd;
+            const int c = part + 8 * i;
+            double value = c == r ? (mine ? diag : 1.0) : 0.0;
+            if (mine && c != r && unknown(c))
+            {
+                if (x > 0 && c == r - 1)
+                    value = -wl;
+                if (x + 1 < l.w && c == r + 1)
+                    value = -wr;
+                if (c == r - l.w)
+                    value = -wu;
+                if (c == r + l.w)
+                    value = -wd;
+            }
+            a[i] = value;
         }
-        a[i] = value;
-    }
+    };
+    form();
 #pragma unroll
     for (int ki = 0; ki < E; ++ki)
     {
@@ -744,8 +890,9 @@ template <typename T> __global__ void __launch_bounds__(kCoarseThreads) k_rebuil
                 pivot_col[buf][r] = a[ki];
             __syncthreads();
             const double pivot = pivot_row[buf][k];
-            if (threadIdx.x == 0 && (!(pivot > 0.0) || !isfinite(pivot)))
-                failed = 1;
+            // (Rows that are no unknown have the pivot one.)
+            if (r == k && mine && !(pivot > kSealedPivot * largest))
+                sealed = 1;
             const double scale = 1.0 / pivot;
             if (r == k)
             {
@@ -766,7 +913,22 @@ template <typename T> __global__ void __launch_bounds__(kCoarseThreads) k_rebuil
             }
         }
     }
-    // C a C over the open cells (the matrix is symmetric: a column's mean is its row's).
+    __syncthreads();
+    const bool exact = sealed != 0;
+    bool failed = false;
+    if (exact)
+    {
+        form();
+        CoarseRow row{{}, r, part};
+#pragma unroll
+        for (int i = 0; i < E; ++i)
+            row.a[i] = a[i];
+        failed = invert_factor(row, diagonal, unknowns, cells);
+#pragma unroll
+        for (int i = 0; i < E; ++i)
+            a[i] = row.a[i];
+    }
+    // Row sums (the matrix is symmetric: a column's is its row's).
     double sum = 0.0;
 #pragma unroll
     for (int i = 0; i < E; ++i)
@@ -778,17 +940,14 @@ template <typename T> __global__ void __launch_bounds__(kCoarseThreads) k_rebuil
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
     sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-    const double share = open_cells > 0 && !dirichlet ? 1.0 / open_cells : 0.0;
+    const double share = open_mask && !dirichlet ? 1.0 / __popcll(open_mask) : 0.0;
+    // C a C over the open cells, unless the solve takes the means.
+    const double fold = exact ? 0.0 : share;
+    const double own_mean = sum * fold;
     if (part == 0)
-        row_mean[r] = sum * share;
+        row_mean[r] = own_mean;
     __syncthreads();
-    if (threadIdx.x < 32)
-    {
-        const double all = warp_sum(row_mean[threadIdx.x] + row_mean[threadIdx.x + 32]);
-        if (threadIdx.x == 0)
-            mean_shared = all * share;
-    }
-    __syncthreads();
+    const double mean = fold * warp_sum(row_mean[lane] + row_mean[lane + 32]);
     if (r < cells)
     {
 #pragma unroll
@@ -798,11 +957,19 @@ template <typename T> __global__ void __launch_bounds__(kCoarseThreads) k_rebuil
             if (c >= cells)
                 continue;
             g.coarse_inverse[r * kTailInverseStride + c] =
-                open[r] && open[c] ? ((a[i] - row_mean[r]) - row_mean[c]) + mean_shared : 0.0;
+                open[r] && open[c] ? ((a[i] - own_mean) - row_mean[c]) + mean : 0.0;
+        }
+        if (part == 0)
+        {
+            g.coarse_inverse[TailMeans::sums(r)] = sum;
+            g.coarse_inverse[TailMeans::open(r)] = open[r];
         }
     }
     if (threadIdx.x == 0)
+    {
+        g.coarse_inverse[TailMeans::share] = share - fold;
         g.state->mg_valid = failed ? 0 : 1;
+    }
 }
 
 } // namespace fc
