@@ -295,6 +295,16 @@ __device__ __forceinline__ FaceMask face_mask(int w, int h, int x, int y, const 
     return m;
 }
 
+// Half the inverse of a face's diagonal, zero for a closed face. Of an infinite diagonal (a viscosity
+// or a mass beyond the working precision) it is no number, not the zero that would close the face:
+// such a solve ends as nonfinite.
+template <typename T> __device__ __forceinline__ T half_inverse(bool open, T diagonal)
+{
+    if (!open)
+        return T(0);
+    return isinf(diagonal) ? T(NAN) : T(0.5) / diagonal;
+}
+
 // Half the inverse diagonal of a level's operator, once per solve: the damped Jacobi sweep is then a
 // multiplication (the two divisions and the face mask were a quarter of its instructions).
 template <typename T>
@@ -312,7 +322,7 @@ __global__ void __launch_bounds__(kViscThreads) k_visc_diagonal(ViscLevel lv, do
     const T4 c = coeff[o.own];
     const T dx = c.z + T(dt) * (T(2) * (c.x + coeff[o.left].x) + c.y + coeff[o.down].y);
     const T dy = c.w + T(dt) * (T(2) * (c.x + coeff[o.up].x) + c.y + coeff[o.right].y);
-    static_cast<T2*>(half)[n] = T2{m.u ? T(0.5) / dx : T(0), m.v ? T(0.5) / dy : T(0)};
+    static_cast<T2*>(half)[n] = T2{half_inverse(m.u, dx), half_inverse(m.v, dy)};
 }
 
 __device__ __forceinline__ bool visc_stopped(const ViscState* s) { return s->stopped || s->breakdown; }

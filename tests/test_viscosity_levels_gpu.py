@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from fluidsim_b200 import FluidGrid, FluidGridState
+from fluidsim_b200._native import FluidCudaError
 
 pytestmark = pytest.mark.gpu
 
@@ -65,3 +66,23 @@ def test_tall_thin_lattice_equals_its_transpose():
         out.append((s.v.T, s.u.T) if transpose else (s.u, s.v))
     for a, b in zip(*out):
         assert np.abs(a - b).max() <= 1e-8 * max(np.abs(b).max(), 1e-30)
+
+
+@pytest.mark.parametrize("precision,viscosity,mass", [("fp32", 1e39, 1.0), ("fp32", 1e38, 1.0), ("fp64", 2.0, np.inf),
+                                                      ("fp32", 2.0, 1e39)])
+def test_a_diagonal_beyond_the_precision_is_an_error(precision, viscosity, mass):
+    """A cell viscosity, a sum of them, or a face mass that overflows: the solve reports it and leaves
+    the velocities (an open face whose inverse diagonal is zero must not count as a closed one)."""
+    w, h = 24, 17
+    rng = np.random.default_rng(1)
+    u, v = rng.uniform(-1, 1, (h, w + 1)), rng.uniform(-1, 1, (h + 1, w))
+    masses = np.ones((h, w))
+    masses[5:9, 3:8] = mass
+    g = FluidGrid(w, h, 1.0, precision)
+    g.configureMaterials([1.0], [1.0], [viscosity], [0.0])
+    g.upload(FluidGridState(np.ones((h, w)), u, v, None, [masses], [np.zeros((h, w))]))
+    before = g.download()
+    with pytest.raises(FluidCudaError):
+        g.applyViscosity(1.0, 1e-4)
+    after = g.download()
+    assert np.array_equal(before.u, after.u) and np.array_equal(before.v, after.v)
