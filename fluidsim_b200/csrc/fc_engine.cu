@@ -166,6 +166,25 @@ void launch_dependent(const char* name, void (*kernel)(Params...), Blocks blocks
         }                                                                                                            \
     } while (0)
 
+// Opts a kernel in to more dynamic shared memory than the default limit, once per device: the
+// attribute belongs to the current device's copy of the kernel. One object per kernel.
+struct SharedOptIn
+{
+    std::atomic<bool> done[64] = {};
+
+    template <typename Kernel> void operator()(Kernel kernel, size_t bytes, const char* what)
+    {
+        int device = 0;
+        check(cudaGetDevice(&device), "device");
+        const bool known = device >= 0 && device < 64;
+        if (known && done[device].load(std::memory_order_acquire))
+            return;
+        check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)), what);
+        if (known)
+            done[device].store(true, std::memory_order_release);
+    }
+};
+
 int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // ------------------------------------------------------------------------------------------
@@ -1301,13 +1320,8 @@ void launch_smooth_kernel(Plan& p, const Range& r, int level, int set, bool depe
     if (r.count <= 0)
         return;
     auto kernel = PRE ? k_smooth_pre<T, K, W, WARPS> : k_smooth_post<T, K, W, WARPS>;
-    static const bool configured = [&]
-    {
-        check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(St::bytes)),
-            "smoothing shared memory");
-        return true;
-    }();
-    (void)configured;
+    static SharedOptIn opt_in;
+    opt_in(kernel, St::bytes, "smoothing shared memory");
     // Resident CTAs: two per SM for 8-warp FP32 regions, one otherwise.
     const int ctas = std::min(r.count, smoothing_ctas(sizeof(T) == 8 || WARPS > 8));
     if (dependent)
@@ -1361,13 +1375,8 @@ template <typename T> void launch_smooth(Plan& p, int level, bool pre, bool depe
 template <typename T, int kThreads> void launch_tail_kernel(Plan& p, bool dependent, cudaStream_t s)
 {
     auto kernel = k_mg_tail<T, kThreads>;
-    static const bool configured = [&]
-    {
-        check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTailMaxBytes)),
-            "tail shared memory");
-        return true;
-    }();
-    (void)configured;
+    static SharedOptIn opt_in;
+    opt_in(kernel, kTailMaxBytes, "tail shared memory");
     if (dependent)
         FC_LAUNCH_DEP(kernel, p.n(), kThreads, p.tail_smem, s, p.d_desc);
     else
@@ -2112,13 +2121,8 @@ ViscWork viscosity_workspace(Grid& g, cudaStream_t s)
 
 template <typename T> void launch_viscosity_tail(ViscWork& w, size_t l, double dt, cudaStream_t s)
 {
-    static const bool configured = [&]
-    {
-        check(cudaFuncSetAttribute(k_visc_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kViscTailMaxBytes)),
-            "viscosity tail shared memory");
-        return true;
-    }();
-    (void)configured;
+    static SharedOptIn opt_in;
+    opt_in(k_visc_tail<T>, kViscTailMaxBytes, "viscosity tail shared memory");
     ViscTail t{};
     int nodes = 0;
     for (size_t k = l; k < w.lev.size(); ++k)
