@@ -41,8 +41,11 @@ constexpr int kShortTileY = 4 * kShortCells;
 // and with short tiles, FP32: 512 x 512 (64 tall tiles) 3491 -> 3089 us, 704 x 704 (121) 3625 ->
 // 3465, 768 x 768 (144) 4774 -> 4493, 832 x 832 (169) 4983 -> 5067, 1024 x 1024 (256) 4963 -> 5319;
 // FP64: 704 x 704 3973 -> 3940, 832 x 832 5337 -> 5528. The rule looks at the grid alone, so a
-// grid's sums do not depend on what else is in its batch.
+// grid's sums do not depend on what else is in its batch. In a plan whose short tiles would fill the
+// SMs many times over (kGroupLimit) a CTA takes a group of four, as tall as a tall tile, and keeps their
+// sums apart.
 constexpr int kShortTileLimit = 148; // tall tiles, one per SM
+constexpr int kGroup = kTallCells / kShortCells;
 inline int vec_cells(int W, int H)
 {
     const long long tall = (long long)((W + kVecTileX - 1) / kVecTileX) * ((H + kTallTileY - 1) / kTallTileY);
@@ -218,8 +221,23 @@ __device__ __forceinline__ double warp_max(double v)
     return v;
 }
 
-// Block reduction of up to four doubles; lane (component) c is summed, or maxed when
-// (max_mask >> c) & 1. Result valid in thread 0. Fixed order: deterministic.
+// Folds the warps' slots in warp order; component c is summed, or maxed when (max_mask >> c) & 1.
+template <int WARPS> __device__ __forceinline__ double4 fold_slots(const double4* slots, int max_mask)
+{
+    double4 out = slots[0];
+    for (int w = 1; w < WARPS; ++w)
+    {
+        const double4 s = slots[w];
+        out.x = (max_mask & 1) ? fmax(out.x, s.x) : out.x + s.x;
+        out.y = (max_mask & 2) ? fmax(out.y, s.y) : out.y + s.y;
+        out.z = (max_mask & 4) ? fmax(out.z, s.z) : out.z + s.z;
+        out.w = (max_mask & 8) ? fmax(out.w, s.w) : out.w + s.w;
+    }
+    return out;
+}
+
+// Block reduction of up to four doubles (fold_slots). Result valid in thread 0. Fixed order:
+// deterministic.
 template <int NT> __device__ double4 block_reduce4(double4 v, int max_mask)
 {
     __shared__ double4 slots[NT / 32];
@@ -232,20 +250,18 @@ template <int NT> __device__ double4 block_reduce4(double4 v, int max_mask)
     if (lane == 0)
         slots[warp] = make_double4(a[0], a[1], a[2], a[3]);
     __syncthreads();
-    double4 out = make_double4(0, 0, 0, 0);
-    if (threadIdx.x == 0)
-    {
-        out = slots[0];
-        for (int w = 1; w < NT / 32; ++w)
-        {
-            const double4 s = slots[w];
-            out.x = (max_mask & 1) ? fmax(out.x, s.x) : out.x + s.x;
-            out.y = (max_mask & 2) ? fmax(out.y, s.y) : out.y + s.y;
-            out.z = (max_mask & 4) ? fmax(out.z, s.z) : out.z + s.z;
-            out.w = (max_mask & 8) ? fmax(out.w, s.w) : out.w + s.w;
-        }
-    }
-    return out;
+    return threadIdx.x == 0 ? fold_slots<NT / 32>(slots, max_mask) : make_double4(0, 0, 0, 0);
+}
+
+// One warp's part of block_reduce4's first N components into its slot.
+template <int N> __device__ __forceinline__ void reduce_to_slot(double4* slots, double4 v, int max_mask)
+{
+    double a[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int c = 0; c < N; ++c)
+        a[c] = ((max_mask >> c) & 1) ? warp_max(a[c]) : warp_sum(a[c]);
+    if ((threadIdx.x & 31) == 0)
+        slots[threadIdx.x >> 5] = make_double4(a[0], a[1], a[2], a[3]);
 }
 
 // The last block's fold of a grid's per-tile partials, in tile order (deterministic): each
@@ -312,17 +328,22 @@ __device__ bool arrive_last(const GridDesc& g, int tile_index, int tiles, double
     return true;
 }
 
-// Arrival of a persistent kernel's run of `run_tiles` tiles of one grid whose partials thread 0
-// already wrote to g.partial[tile]: the CTA counts the run once instead of once per tile, and
-// the last CTA to arrive folds all `tiles` partials (fold_partials). Must be called by all
+// Arrival of a persistent kernel's run of `run_tiles` tiles of one grid whose partials the first
+// WRITERS threads already wrote to g.partial[tile]: the CTA counts the run once instead of once per
+// tile, and the last CTA to arrive folds all `tiles` partials (fold_partials). Must be called by all
 // threads of the block.
-template <int NT>
+template <int NT, int WRITERS = 1>
 __device__ bool arrive_count(const GridDesc& g, int run_tiles, int tiles, double4* total, int max_mask)
 {
     __shared__ int is_last;
+    if (threadIdx.x < 32)
+    {
+        if (threadIdx.x < WRITERS)
+            __threadfence(); // the partials before the count
+        __syncwarp();
+    }
     if (threadIdx.x == 0)
     {
-        __threadfence(); // the partials before the count
         const unsigned int ticket = atomicAdd(g.counter, unsigned(run_tiles));
         is_last = ticket + unsigned(run_tiles) == unsigned(tiles);
     }
@@ -332,6 +353,51 @@ __device__ bool arrive_count(const GridDesc& g, int run_tiles, int tiles, double
     __threadfence();
     fold_partials<NT>(g, tiles, total, max_mask);
     return true;
+}
+
+// Sum tiles of a vector tile (GridDesc::vec_tiles): a grouped tile holds up to kGroup short ones below
+// one another, a row of tiles apart in index; any other tile is one.
+__device__ __forceinline__ int sum_tile_stride(const GridDesc& g) { return (g.W + kVecTileX - 1) / kVecTileX; }
+template <int GROUP> __device__ __forceinline__ int sum_tiles(const GridDesc& g, const Tile& t)
+{
+    return GROUP == 1 ? 1 : min(GROUP, (g.H - t.y0 + kShortTileY - 1) / kShortTileY);
+}
+
+// Partials of a grouped tile's sum tiles from their warps' slots. Must be called by all threads of
+// the block.
+template <int NT, int GROUP>
+__device__ __forceinline__ int write_partials(const GridDesc& g, const Tile& t, const double4 (&slots)[GROUP][NT / 32], int max_mask)
+{
+    __syncthreads();
+    const int count = sum_tiles<GROUP>(g, t);
+    if (int(threadIdx.x) < count)
+        g.partial[t.index + int(threadIdx.x) * sum_tile_stride(g)] = fold_slots<NT / 32>(slots[threadIdx.x], max_mask);
+    return count;
+}
+
+template <int NT, int GROUP>
+__device__ bool arrive_slots(const GridDesc& g, const Tile& t, const double4 (&slots)[GROUP][NT / 32], double4* total, int max_mask)
+{
+    const int count = write_partials<NT, GROUP>(g, t, slots, max_mask);
+    return arrive_count<NT, GROUP>(g, count, g.vec_tiles, total, max_mask);
+}
+
+// Arrival of a vector tile with the partials of its sum tiles, of N components each: the same
+// partials in the same slots, whether a CTA holds one short tile or a group of them, so a grid's sums
+// do not depend on its tiles' launch. Must be called by all threads of the block.
+template <int NT, int N, int GROUP>
+__device__ bool arrive_tile(const GridDesc& g, const Tile& t, const double4 (&mine)[GROUP], double4* total, int max_mask)
+{
+    if constexpr (GROUP == 1)
+        return arrive_last<NT>(g, t.index, g.vec_tiles, block_reduce4<NT>(mine[0], max_mask), total, max_mask);
+    else
+    {
+        __shared__ double4 slots[GROUP][NT / 32];
+#pragma unroll
+        for (int s = 0; s < GROUP; ++s)
+            reduce_to_slot<N>(slots[s], mine[s], max_mask);
+        return arrive_slots<NT, GROUP>(g, t, slots, total, max_mask);
+    }
 }
 
 // Arrival of a persistent kernel's run of `run_tiles` tiles of one grid whose partial pairs are

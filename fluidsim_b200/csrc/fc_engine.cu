@@ -149,21 +149,21 @@ void launch_dependent(const char* name, void (*kernel)(Params...), Blocks blocks
 #define FC_LAUNCH_DEP(kernel, blocks, threads, smem, stream, ...) \
     launch_dependent(#kernel, kernel, (blocks), (threads), (smem), (stream), __VA_ARGS__)
 
-// Launches a vector kernel (a template on CELLS) over the plan's tall and short tiles; `launch` is
-// FC_LAUNCH or FC_LAUNCH_DEP, and a kernel name with commas goes in parentheses.
-#define FC_LAUNCH_VEC(launch, kernel, p, stream, ...)                                                                 \
+// Launches a vector kernel (a template on CELLS and, if it sums, SUM) over the plan's tall tiles, its
+// short ones and its grouped ones; `launch` is FC_LAUNCH or FC_LAUNCH_DEP, and a kernel name with
+// commas goes in parentheses.
+#define FC_LAUNCH_VEC_TILES(launch, kernel, p, set, stream, cells, sum, ...)                                                  \
+    if ((p).vec[set].count > 0)                                                                                      \
+    {                                                                                                                \
+        [[maybe_unused]] constexpr int CELLS = cells, SUM = sum;                                                     \
+        launch(kernel, (p).vec[set].count, ::fc::kVecThreads, 0, stream, (p).d_desc, (p).at((p).vec[set]), ##__VA_ARGS__); \
+    }
+#define FC_LAUNCH_VEC(launch, kernel, p, stream, ...)                                                                        \
     do                                                                                                               \
     {                                                                                                                \
-        if ((p).vec[0].count > 0)                                                                                    \
-        {                                                                                                            \
-            constexpr int CELLS = ::fc::kTallCells;                                                                  \
-            launch(kernel, (p).vec[0].count, ::fc::kVecThreads, 0, stream, (p).d_desc, (p).at((p).vec[0]), ##__VA_ARGS__); \
-        }                                                                                                            \
-        if ((p).vec[1].count > 0)                                                                                    \
-        {                                                                                                            \
-            constexpr int CELLS = ::fc::kShortCells;                                                                 \
-            launch(kernel, (p).vec[1].count, ::fc::kVecThreads, 0, stream, (p).d_desc, (p).at((p).vec[1]), ##__VA_ARGS__); \
-        }                                                                                                            \
+        FC_LAUNCH_VEC_TILES(launch, kernel, p, ::fc::kVecTall, stream, ::fc::kTallCells, ::fc::kTallCells, ##__VA_ARGS__)   \
+        FC_LAUNCH_VEC_TILES(launch, kernel, p, ::fc::kVecShort, stream, ::fc::kShortCells, ::fc::kShortCells, ##__VA_ARGS__) \
+        FC_LAUNCH_VEC_TILES(launch, kernel, p, ::fc::kVecGrouped, stream, ::fc::kTallCells, ::fc::kShortCells, ##__VA_ARGS__) \
     } while (0)
 
 // Opts a kernel in to more dynamic shared memory than the default limit, once per device: the
@@ -839,7 +839,7 @@ __global__ void k_init_states(const GridDesc* grids, int n, const ProjectParams*
 }
 
 // Open (non-solid) cells define the mean-free subspace of the solve.
-template <int CELLS>
+template <int CELLS, int SUM>
 __global__ void __launch_bounds__(kVecThreads) k_count_open(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
@@ -848,16 +848,17 @@ __global__ void __launch_bounds__(kVecThreads) k_count_open(const GridDesc* __re
     if (!g.solid || g.air)
         return;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    double open = 0.0;
+    double4 acc[CELLS / SUM] = {};
+#pragma unroll
     for (int k = 0; k < CELLS; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x >= g.W || y >= g.H)
             continue;
-        open += g.solid[(long long)y * g.W + x] ? 0.0 : 1.0;
+        acc[k / SUM].x += g.solid[(long long)y * g.W + x] ? 0.0 : 1.0;
     }
     __shared__ double4 total;
-    if (arrive_last<kVecThreads>(g, t.index, g.vec_tiles, block_reduce4<kVecThreads>(make_double4(open, 0, 0, 0), 0), &total, 0))
+    if (arrive_tile<kVecThreads, 1>(g, t, acc, &total, 0))
     {
         if (threadIdx.x == 0)
             g.state->inv_cells = total.x > 0.0 ? 1.0 / total.x : 0.0;
@@ -1034,6 +1035,23 @@ __global__ void k_classify(const GridDesc* grids, const Tile* tiles, const doubl
     }
 }
 
+// A plan's vector tiles: of the grids that take tall ones, and of the others, whose short tiles are
+// launched each by itself or, in a crowded plan, in groups of kGroup (vec_cells).
+enum VecSet
+{
+    kVecTall,
+    kVecShort,
+    kVecGrouped,
+    kVecSets
+};
+
+// A plan with more groups than this (two per SM) launches its short tiles in groups: every SM has work
+// without the short tiles' four times as many CTAs, each with its own reduction. Batched FP32
+// projections of uneven grids, short tiles alone and grouped: 144 groups (16 grids) 1.98 and 2.19 ms,
+// 239 (32) 2.90 and 3.03, 358 (24 larger ones) 4.86 and 4.86, 456 (64) 4.57 and 4.45, 4277 (256)
+// 50.4 and 39.4, 8695 (256, with 2918 tall tiles of larger grids) 118.2 and 96.8.
+constexpr int kGroupLimit = 296;
+
 struct Plan
 {
     std::vector<Grid*> grids;
@@ -1048,10 +1066,7 @@ struct Plan
     SolveState* d_states = nullptr;
     SolveState* h_states = nullptr;
     int* d_body_count = nullptr;
-    // Vector tiles of the grids that take tall ones ([0]) and short ones ([1]); consecutive, so that
-    // vec_all covers both.
-    Range vec[2];
-    Range vec_all;
+    Range vec[kVecSets]; // vector tiles, by VecSet
     Range cells; // short tiles over every grid's cells
     Range faces; // short tiles over the (W+1) x (H+1) face index space
     Range pre[kMaxLevels];
@@ -1096,6 +1111,8 @@ struct Plan
     }
 
     const Tile* at(const Range& r) const { return d_tiles + r.offset; }
+    // The tall and the short tiles, which follow one another.
+    Range single_tiles() const { return {vec[kVecTall].offset, vec[kVecTall].count + vec[kVecShort].count}; }
     int n() const { return int(grids.size()); }
 };
 
@@ -1176,15 +1193,27 @@ std::unique_ptr<Plan> make_plan(const std::vector<Grid*>& grids, cudaStream_t st
         body();
         r.count = int(tiles.size()) - r.offset;
     };
-    for (int shape = 0; shape < 2; ++shape)
-        add(plan->vec[shape], [&]
+    long long groups = 0; // of the grids of short tiles
+    for (const Grid* g : grids)
+        if (vec_cells(g->W, g->H) == kShortCells)
+            groups += (long long)ceil_div(g->W, kVecTileX) * ceil_div(g->H, kTallTileY);
+    const VecSet short_set = groups > kGroupLimit ? kVecGrouped : kVecShort;
+    for (const VecSet set : {kVecTall, short_set})
+        add(plan->vec[set], [&]
         {
-            const int cells = shape == 0 ? kTallCells : kShortCells;
+            const int cells = set == kVecTall ? kTallCells : kShortCells;
             for (int i = 0; i < n; ++i)
-                if (vec_cells(grids[i]->W, grids[i]->H) == cells)
-                    append_tiles(tiles, i, grids[i]->W, grids[i]->H, kVecTileX, 4 * cells);
+            {
+                if (vec_cells(grids[i]->W, grids[i]->H) != cells)
+                    continue;
+                const size_t first = tiles.size();
+                append_tiles(tiles, i, grids[i]->W, grids[i]->H, kVecTileX, set == kVecShort ? kShortTileY : kTallTileY);
+                // A group carries the index of its first sum tile.
+                if (set == kVecGrouped)
+                    for (size_t k = first; k < tiles.size(); ++k)
+                        tiles[k].index = tiles[k].y0 / kShortTileY * ceil_div(grids[i]->W, kVecTileX) + tiles[k].x0 / kVecTileX;
+            }
         });
-    plan->vec_all = {plan->vec[0].offset, plan->vec[0].count + plan->vec[1].count};
     add(plan->cells, [&]
     {
         for (int i = 0; i < n; ++i)
@@ -1399,7 +1428,7 @@ template <typename T> void launch_precondition(Plan& p, bool use_mg)
     cudaStream_t s = p.stream;
     if (!use_mg)
     {
-        FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_precondition_diagonal<T, CELLS>), p, s);
+        FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_precondition_diagonal<T, CELLS, SUM>), p, s);
         return;
     }
     for (int l = 0; l < p.max_tail; ++l)
@@ -1409,13 +1438,24 @@ template <typename T> void launch_precondition(Plan& p, bool use_mg)
         launch_smooth<T>(p, l, false, true, s);
 }
 
+// The update of every grid: its persistent CTAs walk tall and short tiles alike, grouped ones apart.
+template <typename T> void launch_update(Plan& p, int parity)
+{
+    const int ctas = kUpdateCtasPerSm * sm_count();
+    const Range each = p.single_tiles();
+    FC_LAUNCH_DEP((k_update<T, 1>), std::min(each.count, ctas), kVecThreads, 0, p.stream, p.d_desc, p.at(each), each.count,
+        parity);
+    const Range& grouped = p.vec[kVecGrouped];
+    FC_LAUNCH_DEP((k_update<T, kGroup>), std::min(grouped.count, ctas), kVecThreads, 0, p.stream, p.d_desc, p.at(grouped),
+        grouped.count, parity);
+}
+
 template <typename T> void launch_iteration(Plan& p, bool use_mg, int parity)
 {
     cudaStream_t s = p.stream;
-    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_direction_operator<T, CELLS>), p, s, parity);
-    FC_LAUNCH_DEP(k_update<T>, std::min(p.vec_all.count, kUpdateCtasPerSm * sm_count()), kVecThreads, 0, s, p.d_desc,
-        p.at(p.vec_all), p.vec_all.count, parity);
-    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_true_residual<T, CELLS>), p, s, 0);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_direction_operator<T, CELLS, SUM>), p, s, parity);
+    launch_update<T>(p, parity);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_true_residual<T, CELLS, SUM>), p, s, 0);
     launch_precondition<T>(p, use_mg);
 }
 
@@ -1425,12 +1465,12 @@ template <typename T> void launch_setup(Plan& p, bool use_mg)
     cudaStream_t s = p.stream;
     // The first launch follows a copy (or starts the graph); the others follow a kernel.
     FC_LAUNCH(k_init_states, ceil_div(p.n(), 128), 128, 0, s, p.d_desc, p.n(), p.d_params, p.d_body_count);
-    FC_LAUNCH_VEC(FC_LAUNCH_DEP, k_count_open<CELLS>, p, s);
-    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_rhs<T, CELLS>), p, s);
-    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_rhs_stats<T, CELLS>), p, s);
-    FC_LAUNCH_VEC(FC_LAUNCH_DEP, k_warm_start<CELLS>, p, s);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_count_open<CELLS, SUM>), p, s);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_rhs<T, CELLS, SUM>), p, s);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_rhs_stats<T, CELLS, SUM>), p, s);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_warm_start<CELLS, SUM>), p, s);
     FC_LAUNCH_VEC(FC_LAUNCH_DEP, k_remove_pressure_mean<CELLS>, p, s);
-    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_true_residual<T, CELLS>), p, s, 1);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_true_residual<T, CELLS, SUM>), p, s, 1);
     launch_precondition<T>(p, use_mg);
 }
 
@@ -1440,11 +1480,13 @@ template <typename T> void launch_finish(Plan& p)
     cudaStream_t s = p.stream;
     // The first launch follows the loop (a conditional node in the graph); the others follow a
     // kernel.
-    FC_LAUNCH(k_flush_pressure<T>, p.vec_all.count, kVecThreads, 0, s, p.d_desc, p.at(p.vec_all));
-    FC_LAUNCH_VEC(FC_LAUNCH_DEP, k_pressure_sum<CELLS>, p, s);
+    const Range each = p.single_tiles();
+    FC_LAUNCH((k_flush_pressure<T, 1>), each.count, kVecThreads, 0, s, p.d_desc, p.at(each));
+    FC_LAUNCH((k_flush_pressure<T, kGroup>), p.vec[kVecGrouped].count, kVecThreads, 0, s, p.d_desc, p.at(p.vec[kVecGrouped]));
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_pressure_sum<CELLS, SUM>), p, s);
     FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_velocity_update<T, CELLS>), p, s);
     FC_LAUNCH_VEC(FC_LAUNCH_DEP, k_remove_pressure_mean<CELLS>, p, s);
-    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_divergence<T, CELLS>), p, s);
+    FC_LAUNCH_VEC(FC_LAUNCH_DEP, (k_divergence<T, CELLS, SUM>), p, s);
     FC_LAUNCH_DEP(k_gather_states, ceil_div(p.n(), 128), 128, 0, s, p.d_desc, p.n(), p.d_states);
 }
 
@@ -2476,7 +2518,7 @@ double time_kernel(Grid& g, int kernel, int repeats)
             {
             case 0: launch_smooth<T>(p, 0, true, false, p.stream); break;
             case 1: launch_smooth<T>(p, 0, false, false, p.stream); break;
-            case 2: FC_LAUNCH_VEC(FC_LAUNCH, (k_direction_operator<T, CELLS>), p, p.stream, 0); break;
+            case 2: FC_LAUNCH_VEC(FC_LAUNCH, (k_direction_operator<T, CELLS, SUM>), p, p.stream, 0); break;
             default: launch_tail<T>(p, false, p.stream); break;
             }
         };
@@ -3712,7 +3754,7 @@ int fc_max_divergence(fc_grid* grid, double* out)
         fc::dispatch(g.precision, [&](auto zero)
         {
             using T = decltype(zero);
-            FC_LAUNCH_VEC(FC_LAUNCH, (fc::k_divergence<T, CELLS>), p, p.stream);
+            FC_LAUNCH_VEC(FC_LAUNCH, (fc::k_divergence<T, CELLS, SUM>), p, p.stream);
         });
         fc::SolveState s;
         check(cudaMemcpyAsync(&s, g.desc.state, sizeof(s), cudaMemcpyDeviceToHost, p.stream), "divergence");

@@ -42,7 +42,7 @@ __device__ __forceinline__ void finish_preconditioner(SolveState& s, double sum_
 }
 
 // Diagonal (Jacobi) preconditioner: z = (r - mean r) / diag. FluidGridCPU.cpp:1691-1698.
-template <typename T, int CELLS>
+template <typename T, int CELLS, int SUM>
 __global__ void __launch_bounds__(kVecThreads) k_precondition_diagonal(const GridDesc* grids, const Tile* tiles)
 {
     allow_dependents();
@@ -58,7 +58,8 @@ __global__ void __launch_bounds__(kVecThreads) k_precondition_diagonal(const Gri
     const T* r = static_cast<const T*>(g.r);
     T* z = static_cast<T*>(g.z);
     const double mean_r = s.mean_r;
-    double sz = 0.0, srz = 0.0;
+    double4 acc[CELLS / SUM] = {};
+#pragma unroll
     for (int k = 0; k < CELLS; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
@@ -71,11 +72,11 @@ __global__ void __launch_bounds__(kVecThreads) k_precondition_diagonal(const Gri
         z[i] = value;
         if (g.solid && g.solid[(long long)y * g.W + x])
             continue;
-        sz += double(value);
-        srz += double(r[i]) * double(value);
+        acc[k / SUM].x += double(value);
+        acc[k / SUM].y += double(r[i]) * double(value);
     }
     __shared__ double4 total;
-    if (arrive_last<kVecThreads>(g, t.index, g.vec_tiles, block_reduce4<kVecThreads>(make_double4(sz, srz, 0, 0), 0), &total, 0))
+    if (arrive_tile<kVecThreads, 2>(g, t, acc, &total, 0))
     {
         if (threadIdx.x == 0)
             finish_preconditioner(s, total.x, total.y);

@@ -3,6 +3,7 @@
 // Every kernel takes the grid descriptors and a tile table, so one launch serves one grid or a
 // batch of independent grids of uneven sizes (each CTA looks up its grid). A tile is 64 columns and
 // 4 CELLS rows (64 or 16, by the grid's size; vec_cells), worked by 256 threads of CELLS cells each.
+// Its sums are those of sum tiles of 4 SUM rows: the whole tile, or (CELLS 16, SUM 4) four short ones.
 // Reductions are folded in FP64: each CTA writes one
 // partial and the last CTA of a grid to arrive folds them in tile order, so results do not
 // depend on which other grids share the launch.
@@ -185,7 +186,7 @@ __device__ __forceinline__ void cell_faces(T* __restrict__ u, T* __restrict__ v,
 
 // b = -(du + dv)/dx * dx^2/dt with closed faces zeroed; sums b over open cells.
 // FluidGridCPU.cpp:1050-1083.
-template <typename T, int CELLS> __global__ void __launch_bounds__(kVecThreads) k_rhs(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
+template <typename T, int CELLS, int SUM> __global__ void __launch_bounds__(kVecThreads) k_rhs(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
     FC_VEC_TILE_PROLOGUE
@@ -198,7 +199,7 @@ template <typename T, int CELLS> __global__ void __launch_bounds__(kVecThreads) 
     const unsigned char* __restrict__ solid = g.solid;
     const unsigned char* __restrict__ air = g.air;
     double* __restrict__ rhs = g.b;
-    double sum = 0.0;
+    double4 acc[CELLS / SUM] = {};
 #pragma unroll
     for (int k = 0; k < CELLS; ++k)
     {
@@ -213,10 +214,10 @@ template <typename T, int CELLS> __global__ void __launch_bounds__(kVecThreads) 
         if (held_at(solid, air, W, x, y))
             b = 0.0;
         rhs[padded_index(S, x, y)] = b;
-        sum += b;
+        acc[k / SUM].x += b;
     }
     __shared__ double4 total;
-    if (arrive_last<kVecThreads>(g, t.index, g.vec_tiles, block_reduce4<kVecThreads>(make_double4(sum, 0, 0, 0), 0), &total, 0))
+    if (arrive_tile<kVecThreads, 1>(g, t, acc, &total, 0))
     {
         if (threadIdx.x == 0)
             g.state->mean_b = total.x * g.state->inv_cells;
@@ -224,7 +225,7 @@ template <typename T, int CELLS> __global__ void __launch_bounds__(kVecThreads) 
 }
 
 // max |b - mean| and sum (b - mean)^2; decides the early exit (FluidGridCPU.cpp:1731-1740).
-template <typename T, int CELLS> __global__ void __launch_bounds__(kVecThreads) k_rhs_stats(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
+template <typename T, int CELLS, int SUM> __global__ void __launch_bounds__(kVecThreads) k_rhs_stats(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
     FC_VEC_TILE_PROLOGUE
@@ -233,7 +234,7 @@ template <typename T, int CELLS> __global__ void __launch_bounds__(kVecThreads) 
     const unsigned char* __restrict__ solid = g.solid;
     const unsigned char* __restrict__ air = g.air;
     const double* __restrict__ rhs = g.b;
-    double mx = 0.0, sq = 0.0;
+    double4 acc[CELLS / SUM] = {};
 #pragma unroll
     for (int k = 0; k < CELLS; ++k)
     {
@@ -241,11 +242,12 @@ template <typename T, int CELLS> __global__ void __launch_bounds__(kVecThreads) 
         if (x >= W || y >= H || held_at(solid, air, W, x, y))
             continue;
         const double b = rhs[padded_index(S, x, y)] - mean;
-        mx = fmax(mx, isfinite(b) ? fabs(b) : INFINITY);
-        sq += b * b;
+        double4& a = acc[k / SUM];
+        a.x = fmax(a.x, isfinite(b) ? fabs(b) : INFINITY);
+        a.y += b * b;
     }
     __shared__ double4 total;
-    if (arrive_last<kVecThreads>(g, t.index, g.vec_tiles, block_reduce4<kVecThreads>(make_double4(mx, sq, 0, 0), 1), &total, 1))
+    if (arrive_tile<kVecThreads, 2>(g, t, acc, &total, 1))
     {
         if (threadIdx.x == 0)
         {
@@ -265,7 +267,7 @@ template <typename T, int CELLS> __global__ void __launch_bounds__(kVecThreads) 
 
 // Warm start p = 2p - p_prev, or clear both when no solve is needed; sums the prediction.
 // FluidGridCPU.cpp:1731-1753.
-template <int CELLS> __global__ void __launch_bounds__(kVecThreads) k_warm_start(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
+template <int CELLS, int SUM> __global__ void __launch_bounds__(kVecThreads) k_warm_start(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
     FC_VEC_TILE_PROLOGUE
@@ -275,7 +277,7 @@ template <int CELLS> __global__ void __launch_bounds__(kVecThreads) k_warm_start
     const unsigned char* __restrict__ air = g.air;
     double* __restrict__ p = g.p;
     double* __restrict__ p_prev = g.p_prev;
-    double sum = 0.0;
+    double4 acc[CELLS / SUM] = {};
 #pragma unroll
     for (int k = 0; k < CELLS; ++k)
     {
@@ -293,10 +295,10 @@ template <int CELLS> __global__ void __launch_bounds__(kVecThreads) k_warm_start
         const double predicted = 2.0 * latest - p_prev[i];
         p[i] = predicted;
         p_prev[i] = latest;
-        sum += predicted;
+        acc[k / SUM].x += predicted;
     }
     __shared__ double4 total;
-    if (arrive_last<kVecThreads>(g, t.index, g.vec_tiles, block_reduce4<kVecThreads>(make_double4(sum, 0, 0, 0), 0), &total, 0))
+    if (arrive_tile<kVecThreads, 1>(g, t, acc, &total, 0))
     {
         if (threadIdx.x == 0)
             g.state->mean_p = total.x * g.state->inv_cells;
@@ -304,7 +306,7 @@ template <int CELLS> __global__ void __launch_bounds__(kVecThreads) k_warm_start
 }
 
 // Pressure sum for the final mean removal.
-template <int CELLS> __global__ void __launch_bounds__(kVecThreads) k_pressure_sum(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
+template <int CELLS, int SUM> __global__ void __launch_bounds__(kVecThreads) k_pressure_sum(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
     FC_VEC_TILE_PROLOGUE
@@ -314,17 +316,17 @@ template <int CELLS> __global__ void __launch_bounds__(kVecThreads) k_pressure_s
     const unsigned char* __restrict__ solid = g.solid;
     const unsigned char* __restrict__ air = g.air;
     const double* __restrict__ p = g.p;
-    double sum = 0.0;
+    double4 acc[CELLS / SUM] = {};
 #pragma unroll
     for (int k = 0; k < CELLS; ++k)
     {
         const int x = t.x0 + tx + 32 * (k & 1), y = t.y0 + ty + 8 * (k >> 1);
         if (x >= W || y >= H || held_at(solid, air, W, x, y))
             continue;
-        sum += p[padded_index(S, x, y)];
+        acc[k / SUM].x += p[padded_index(S, x, y)];
     }
     __shared__ double4 total;
-    if (arrive_last<kVecThreads>(g, t.index, g.vec_tiles, block_reduce4<kVecThreads>(make_double4(sum, 0, 0, 0), 0), &total, 0))
+    if (arrive_tile<kVecThreads, 1>(g, t, acc, &total, 0))
     {
         if (threadIdx.x == 0)
             g.state->mean_p = total.x * g.state->inv_cells;
@@ -382,7 +384,7 @@ __device__ __forceinline__ double apply_cell_fp64_pending(const T* right, const 
 // True residual r = (b - mean b) - A p in FP64, stored in the working type, with its stats.
 // `initial` selects the solve's first residual (FluidGridCPU.cpp:1754-1757) versus the
 // convergence check inside the loop (:1795-1804).
-template <typename T, int CELLS>
+template <typename T, int CELLS, int SUM>
 __global__ void __launch_bounds__(kVecThreads) k_true_residual(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles, int initial)
 {
     allow_dependents();
@@ -404,7 +406,7 @@ __global__ void __launch_bounds__(kVecThreads) k_true_residual(const GridDesc* _
     const bool pending = !initial && s.p_pending;
     const T* __restrict__ d0 = static_cast<const T*>(g.d[1]);
     const double alpha0 = s.alpha_pending;
-    double sum = 0.0, mx = 0.0, sq = 0.0;
+    double4 acc[CELLS / SUM] = {};
 #pragma unroll
     for (int k = 0; k < CELLS; ++k)
     {
@@ -419,12 +421,13 @@ __global__ void __launch_bounds__(kVecThreads) k_true_residual(const GridDesc* _
         const T stored = T(value);
         r[i] = stored;
         const double rv = dd(stored);
-        sum += rv;
-        mx = fmax(mx, fabs(rv));
-        sq += rv * rv;
+        double4& a = acc[k / SUM];
+        a.x += rv;
+        a.y = fmax(a.y, fabs(rv));
+        a.z += rv * rv;
     }
     __shared__ double4 total;
-    if (arrive_last<kVecThreads>(g, t.index, g.vec_tiles, block_reduce4<kVecThreads>(make_double4(sum, mx, sq, 0), 2), &total, 2))
+    if (arrive_tile<kVecThreads, 3>(g, t, acc, &total, 2))
     {
         if (threadIdx.x == 0)
         {
@@ -474,20 +477,21 @@ template <> struct VecPair<double>
 };
 
 // d = (z - mean z) + beta d_old; q = A d; d.q through the grid's reduction. Warp w handles
-// CELLS / 2 rows of the tile's 64 columns (lane = column pair) in passes of two rows: all
+// SUM / 2 rows of each sum tile's 64 columns (lane = column pair) in passes of two rows: all
 // loads of a pass (four rows of z and d, two rows of weights) are issued first, then the
 // directions and the operator are formed in registers; horizontal neighbours across pairs are
 // warp shuffles, and lanes 0 and 31 fetch the columns just outside the warp. At 64 registers
 // four CTAs fit an SM in FP32, which hides more load latency than passes of four rows at 80
 // registers and three CTAs (31.5 -> 30.2 us at 2048 x 2048).
 // Operator: FluidGridCPU.cpp:1507-1598.
-template <typename T, int CELLS>
+template <typename T, int CELLS, int SUM>
 __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? 4 : 1)
     k_direction_operator(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles, int parity)
 {
     using P = typename VecPair<T>::type;
     constexpr int R = 2;
-    constexpr int ROWS = CELLS / 2; // of each warp
+    constexpr int ROWS = SUM / 2; // of each warp in a sum tile
+    constexpr int GROUP = CELLS / SUM;
     allow_dependents();
     const Tile t = tiles[blockIdx.x];
     const GridDesc& g = grids[t.grid];
@@ -509,10 +513,15 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? 4 : 1)
     // Column just outside the warp: left of the first pair for lane 0, right of the last for 31.
     const int edge_x = lane == 0 ? gx - 1 : gx + 2;
     const bool edge = (lane == 0 && cols) || (lane == 31 && gx + 2 + kPadX < S);
-    // A warp below the grid (a short tile's remainder) has no row above it either.
-    P up_w = P{};
-    if (cols && t.y0 + ROWS * warp <= H)
-        up_w = *reinterpret_cast<const P*>(down + padded_index(S, gx, t.y0 + ROWS * warp - 1));
+    // Weights of the row above y0; a warp below the grid (a short tile's remainder) has none.
+    P up_w;
+    auto load_above = [&](int y0)
+    {
+        up_w = P{};
+        if (cols && y0 <= H)
+            up_w = *reinterpret_cast<const P*>(down + padded_index(S, gx, y0 - 1));
+    };
+    load_above(t.y0 + ROWS * warp);
     // Face weights of two rows, which no kernel of the projection writes: a short tile's only pass has
     // them on their way before the wait.
     P w[R], dn[R];
@@ -539,7 +548,7 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? 4 : 1)
             }
         }
     };
-    constexpr bool kOnePass = ROWS == R;
+    constexpr bool kOnePass = ROWS == R && GROUP == 1;
     if (kOnePass)
         load_weights(t.y0 + ROWS * warp);
     dependency_wait();
@@ -547,11 +556,16 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? 4 : 1)
     if (s.done)
         return;
     const T mz = T(mean_z), b = T(beta);
+    // A grouped tile's sum tiles are the passes: each ends with its sum.
+    static_assert(GROUP == 1 || ROWS == R, "one pass a sum tile of a group");
+    __shared__ double4 slots[GROUP][kVecThreads / 32];
     double dot = 0.0;
 #pragma unroll 1
-    for (int pass = 0; pass < ROWS / R; ++pass)
+    for (int pass = 0; pass < GROUP * ROWS / R; ++pass)
     {
-        const int y0 = t.y0 + ROWS * warp + R * pass;
+        const int y0 = GROUP == 1 ? t.y0 + ROWS * warp + R * pass : t.y0 + kShortTileY * pass + R * warp;
+        if (GROUP > 1 && pass > 0)
+            load_above(y0);
         P zz[R + 2], dd0[R + 2];
         T ez[R], ed[R];
 #pragma unroll
@@ -639,9 +653,19 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? 4 : 1)
             }
         }
         up_w = dn[R - 1];
+        if (GROUP > 1)
+        {
+            reduce_to_slot<1>(slots[pass], make_double4(dot, 0, 0, 0), 0);
+            dot = 0.0;
+        }
     }
     __shared__ double4 total;
-    if (arrive_last<kVecThreads>(g, t.index, g.vec_tiles, block_reduce4<kVecThreads>(make_double4(dot, 0, 0, 0), 0), &total, 0))
+    bool last;
+    if constexpr (GROUP == 1)
+        last = arrive_last<kVecThreads>(g, t.index, g.vec_tiles, block_reduce4<kVecThreads>(make_double4(dot, 0, 0, 0), 0), &total, 0);
+    else
+        last = arrive_slots<kVecThreads, GROUP>(g, t, slots, &total, 0);
+    if (last)
     {
         if (threadIdx.x == 0)
         {
@@ -662,7 +686,7 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? 4 : 1)
 // persistent (two CTAs per SM walk the slices of every grid), each thread takes two quads of
 // four cells per step with every load of the step issued before the arithmetic, and a CTA
 // counts its slices of a grid once; the per-slice partials and their fold are those of one CTA
-// per slice.
+// per slice. A slice is that of a sum tile.
 //
 // The loop runs its iterations in pairs (parity 0, then 1). Nothing inside the loop reads p
 // except the true residual, so the first iteration of a pair updates only r and leaves its
@@ -713,7 +737,10 @@ template <typename T> __device__ __forceinline__ UpdateArgs<T> update_args(const
         static_cast<T*>(g.r), g.p, quads, (quads + g.vec_tiles - 1) / g.vec_tiles};
 }
 
-template <typename T>
+// GROUP short tiles an entry (kGroup in a crowded plan, see vec_cells): an entry's slices are then
+// worked two at a time, so that both have their loads in flight (a slice of a short tile is about one
+// quad a thread), and folded behind one barrier. A slice's sums are formed alike either way.
+template <typename T, int GROUP>
 __global__ void __launch_bounds__(kVecThreads, kUpdateCtasPerSm)
     k_update(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles, int count, int parity)
 {
@@ -721,6 +748,9 @@ __global__ void __launch_bounds__(kVecThreads, kUpdateCtasPerSm)
     // Quads per thread and step (FP64 takes one: its quads are twice the registers). A thread
     // visits the same quads in the same order either way.
     constexpr int U = sizeof(T) == 4 ? 2 : 1;
+    // Slices worked at a time, quads of each, and the distance of a thread's quads in a slice.
+    constexpr int SLICES = GROUP == 1 ? 1 : U;
+    constexpr int STEP = kVecThreads * (U / SLICES);
     allow_dependents();
     // The first slice's entry and descriptor fields are read before the wait.
     int i = blockIdx.x;
@@ -728,7 +758,9 @@ __global__ void __launch_bounds__(kVecThreads, kUpdateCtasPerSm)
     UpdateArgs<T> a = update_args<T>(grids[t.grid], parity);
     dependency_wait();
     __shared__ double4 total;
+    __shared__ double4 slots[2][GROUP][kVecThreads / 32]; // of every other entry
     int run = 0; // slices of the current grid finished since the last count
+    int flip = 0;
     for (; i < count; i += gridDim.x)
     {
         if (i != int(blockIdx.x))
@@ -749,68 +781,97 @@ __global__ void __launch_bounds__(kVecThreads, kUpdateCtasPerSm)
         const bool pending = update_p && s.p_pending;
         const double alpha0 = s.alpha_pending;
         const T* const d0 = a.d0;
-        const int first = min(a.quads, a.per * t.index);
-        const int last = min(a.quads, first + a.per);
-        double sum = 0.0, mx = 0.0, sq = 0.0;
-        for (int base = first + int(threadIdx.x); base < last; base += kVecThreads * U)
+        const int slices = sum_tiles<GROUP>(g, t), stride = GROUP == 1 ? 0 : sum_tile_stride(g);
+        double4 part;
+#pragma unroll 1
+        for (int k0 = 0; k0 < slices; k0 += SLICES)
         {
-            Q dv[U], d0v[U], qv[U], rv[U];
-            double4 pv[U];
+            int first[SLICES], last[SLICES];
+            double sum[SLICES], mx[SLICES], sq[SLICES];
 #pragma unroll
-            for (int u = 0; u < U; ++u)
+            for (int k = 0; k < SLICES; ++k)
             {
-                const int j = base + u * kVecThreads;
-                if (j < last)
+                first[k] = min(a.quads, a.per * (t.index + (k0 + k) * stride));
+                last[k] = k0 + k < slices ? min(a.quads, first[k] + a.per) : first[k];
+                sum[k] = mx[k] = sq[k] = 0.0;
+            }
+            const int longest = GROUP == 1 ? last[0] - first[0] : a.per;
+            for (int base = int(threadIdx.x); base < longest; base += STEP)
+            {
+                Q dv[U], d0v[U], qv[U], rv[U];
+                double4 pv[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
                 {
-                    qv[u] = reinterpret_cast<const Q*>(q)[j];
-                    rv[u] = reinterpret_cast<const Q*>(r)[j];
+                    const int k = u % SLICES;
+                    const int j = first[k] + base + u / SLICES * kVecThreads;
+                    if (j < last[k])
+                    {
+                        qv[u] = reinterpret_cast<const Q*>(q)[j];
+                        rv[u] = reinterpret_cast<const Q*>(r)[j];
+                        if (update_p)
+                        {
+                            dv[u] = reinterpret_cast<const Q*>(d)[j];
+                            pv[u] = reinterpret_cast<const double4*>(a.p)[j];
+                            if (pending)
+                                d0v[u] = reinterpret_cast<const Q*>(d0)[j];
+                        }
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                {
+                    const int k = u % SLICES;
+                    const int j = first[k] + base + u / SLICES * kVecThreads;
+                    if (j >= last[k])
+                        continue;
                     if (update_p)
                     {
-                        dv[u] = reinterpret_cast<const Q*>(d)[j];
-                        pv[u] = reinterpret_cast<const double4*>(a.p)[j];
+                        double4 pp = pv[u];
                         if (pending)
-                            d0v[u] = reinterpret_cast<const Q*>(d0)[j];
+                            add_step<T>(pp, alpha0, d0v[u]);
+                        add_step<T>(pp, alpha, dv[u]);
+                        reinterpret_cast<double4*>(a.p)[j] = pp;
+                    }
+                    Q rr;
+                    rr.x = T(double(rv[u].x) - alpha * double(qv[u].x));
+                    rr.y = T(double(rv[u].y) - alpha * double(qv[u].y));
+                    rr.z = T(double(rv[u].z) - alpha * double(qv[u].z));
+                    rr.w = T(double(rv[u].w) - alpha * double(qv[u].w));
+                    reinterpret_cast<Q*>(r)[j] = rr;
+                    const double e[4] = {double(rr.x), double(rr.y), double(rr.z), double(rr.w)};
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                    {
+                        sum[k] += e[c];
+                        mx[k] = fmax(mx[k], fabs(e[c]));
+                        sq[k] += e[c] * e[c];
                     }
                 }
             }
-#pragma unroll
-            for (int u = 0; u < U; ++u)
+            if constexpr (GROUP == 1)
+                part = block_reduce4<kVecThreads>(make_double4(sum[0], mx[0], sq[0], 0), 2);
+            else
             {
-                const int j = base + u * kVecThreads;
-                if (j >= last)
-                    continue;
-                if (update_p)
-                {
-                    double4 pp = pv[u];
-                    if (pending)
-                        add_step<T>(pp, alpha0, d0v[u]);
-                    add_step<T>(pp, alpha, dv[u]);
-                    reinterpret_cast<double4*>(a.p)[j] = pp;
-                }
-                Q rr;
-                rr.x = T(double(rv[u].x) - alpha * double(qv[u].x));
-                rr.y = T(double(rv[u].y) - alpha * double(qv[u].y));
-                rr.z = T(double(rv[u].z) - alpha * double(qv[u].z));
-                rr.w = T(double(rv[u].w) - alpha * double(qv[u].w));
-                reinterpret_cast<Q*>(r)[j] = rr;
-                const double e[4] = {double(rr.x), double(rr.y), double(rr.z), double(rr.w)};
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
-                {
-                    sum += e[c];
-                    mx = fmax(mx, fabs(e[c]));
-                    sq += e[c] * e[c];
-                }
+                for (int k = 0; k < SLICES; ++k)
+                    if (k0 + k < slices)
+                        reduce_to_slot<3>(slots[flip][k0 + k], make_double4(sum[k], mx[k], sq[k], 0), 2);
             }
         }
-        const double4 part = block_reduce4<kVecThreads>(make_double4(sum, mx, sq, 0), 2);
-        if (threadIdx.x == 0)
-            g.partial[t.index] = part;
-        ++run;
+        if constexpr (GROUP == 1)
+        {
+            if (threadIdx.x == 0)
+                g.partial[t.index] = part;
+        }
+        else
+            write_partials<kVecThreads, GROUP>(g, t, slots[flip], 2);
+        flip ^= 1;
+        run += slices;
         const int next = i + gridDim.x;
         if (next >= count || tiles[next].grid != t.grid)
         {
-            if (arrive_count<kVecThreads>(g, run, g.vec_tiles, &total, 2))
+            if (arrive_count<kVecThreads, GROUP>(g, run, g.vec_tiles, &total, 2))
             {
                 if (threadIdx.x == 0)
                 {
@@ -841,7 +902,7 @@ __global__ void __launch_bounds__(kVecThreads, kUpdateCtasPerSm)
 
 // Applies a pair's pending p += alpha d at the loop's exit (see k_update), over the padded
 // array as one flat stream; p is read only after this.
-template <typename T> __global__ void __launch_bounds__(kVecThreads) k_flush_pressure(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
+template <typename T, int GROUP> __global__ void __launch_bounds__(kVecThreads) k_flush_pressure(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
     using Q = typename Quad<T>::type;
@@ -854,13 +915,17 @@ template <typename T> __global__ void __launch_bounds__(kVecThreads) k_flush_pre
     const double alpha0 = s.alpha_pending;
     const long long quads = (long long)g.S * (g.H + 2) / 4;
     const long long per = (quads + g.vec_tiles - 1) / g.vec_tiles;
-    const long long first = per * t.index;
-    const long long last = min(quads, first + per);
-    for (long long j = first + threadIdx.x; j < last; j += kVecThreads)
+    const int slices = sum_tiles<GROUP>(g, t), stride = GROUP == 1 ? 0 : sum_tile_stride(g);
+    for (int k = 0; k < slices; ++k)
     {
-        double4 pp = reinterpret_cast<const double4*>(g.p)[j];
-        add_step<T>(pp, alpha0, reinterpret_cast<const Q*>(d0)[j]);
-        reinterpret_cast<double4*>(g.p)[j] = pp;
+        const long long first = per * (t.index + k * stride);
+        const long long last = min(quads, first + per);
+        for (long long j = first + threadIdx.x; j < last; j += kVecThreads)
+        {
+            double4 pp = reinterpret_cast<const double4*>(g.p)[j];
+            add_step<T>(pp, alpha0, reinterpret_cast<const Q*>(d0)[j]);
+            reinterpret_cast<double4*>(g.p)[j] = pp;
+        }
     }
 }
 
@@ -924,7 +989,7 @@ __device__ __forceinline__ double face_ulp(double value)
 // max |div u| (FluidGridCPU.cpp:1126-1152), its excess over the float rounding allowance of the
 // four faces (as UniformWebGPU's velocity_stats, FluidUniformWebGPUKernels.h:166-213), and the
 // sum of squares.
-template <typename T, int CELLS> __global__ void __launch_bounds__(kVecThreads) k_divergence(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
+template <typename T, int CELLS, int SUM> __global__ void __launch_bounds__(kVecThreads) k_divergence(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles)
 {
     dependent_start();
     FC_VEC_TILE_PROLOGUE
@@ -935,8 +1000,7 @@ template <typename T, int CELLS> __global__ void __launch_bounds__(kVecThreads) 
     const bool dirichlet = g.air != nullptr;
     const unsigned char* __restrict__ solid = g.solid;
     const double* __restrict__ fraction = g.fraction;
-    double mx = 0.0, excess = 0.0, sq = 0.0;
-    int nonfinite = 0;
+    double4 acc[CELLS / SUM] = {}; // max, excess, square sum, nonfinite
 #pragma unroll
     for (int k = 0; k < CELLS; ++k)
     {
@@ -951,19 +1015,19 @@ template <typename T, int CELLS> __global__ void __launch_bounds__(kVecThreads) 
         const long long iu = (long long)y * (W + 1) + x;
         const T ul = u[iu], ur = u[iu + 1], vu = v[iv], vd = v[iv + W];
         const double div = ((dd(ur) - dd(ul)) + (dd(vd) - dd(vu))) / dx;
+        double4& a = acc[k / SUM];
         if (!isfinite(div))
         {
-            nonfinite = 1;
+            a.w = 1.0;
             continue;
         }
         const double rounding = (face_ulp(ul) + face_ulp(ur) + face_ulp(vu) + face_ulp(vd)) / dx;
-        mx = fmax(mx, fabs(div));
-        excess = fmax(excess, fmax(0.0, fabs(div) - rounding));
-        sq += div * div;
+        a.x = fmax(a.x, fabs(div));
+        a.y = fmax(a.y, fmax(0.0, fabs(div) - rounding));
+        a.z += div * div;
     }
     __shared__ double4 total;
-    const double4 mine = make_double4(mx, excess, sq, double(nonfinite));
-    if (arrive_last<kVecThreads>(g, t.index, g.vec_tiles, block_reduce4<kVecThreads>(mine, 1 | 2 | 8), &total, 1 | 2 | 8))
+    if (arrive_tile<kVecThreads, 4>(g, t, acc, &total, 1 | 2 | 8))
     {
         if (threadIdx.x == 0)
         {

@@ -1,5 +1,5 @@
-"""The fine-level vector kernels' tall and short tiles (vec_cells): grids on both sides of the rule
-project alike alone and together in one batch, and against the FP64 restatement."""
+"""The fine-level vector kernels' tall, short and grouped tiles (vec_cells, kGroupLimit): grids on both
+sides of the rules project alike alone and together in one batch, and against the FP64 restatement."""
 import numpy as np
 import pytest
 
@@ -47,3 +47,36 @@ def test_short_tiles_match_restatement(oracle, size):
     assert r.converged and abs(r.iterations - e.iterations) <= 3
     scale = max(np.abs(u).max(), np.abs(v).max())
     assert np.abs(d.u - u).max() <= 1e-8 * scale and np.abs(d.v - v).max() <= 1e-8 * scale
+
+
+# Grids of short tiles whose groups end after one to four of them, in one column of tiles or several.
+GROUPED = [(64, 64), (65, 65), (130, 49), (1, 300), (90, 17), (33, 128), (200, 97), (70, 145)]
+
+
+@pytest.mark.parametrize("precision,air,preconditioner",
+                         [("fp32", "gas", "multigrid"), ("fp64", "gas", "multigrid"), ("mixed", "dirichlet", "multigrid"),
+                          ("fp32", "gas", "diagonal")])
+def test_crowded_batch_equals_single(precision, air, preconditioner):
+    """More than 296 groups of short tiles, and a grid of tall ones: every sum of a grid is formed as
+    when it is alone, so the batch equals the grids bit for bit."""
+    members = [scenes.random_pool(w, h, seed=i, fill=0.55, obstacles=i % 3) for i, (w, h) in enumerate(GROUPED * 12)]
+    members.append(scenes.random_pool(832, 769, seed=1, fill=0.55))
+    assert sum(-(-s.width // 64) * -(-s.height // 64) for s in members[:-1]) > 296
+    for s in members:
+        s.air_model = air
+    cap = 300 if preconditioner == "multigrid" else 20
+    batch_grids = [_grid(s, precision) for s in members]
+    for g in batch_grids:
+        g.setPreconditioner(preconditioner)
+    batch = ProjectionBatch(batch_grids)
+    together = batch.project([s.dt for s in members], cap, 1e-6, relative_tolerance=1e-6)
+    for s, g, r in zip(members, batch_grids, together):
+        alone = _grid(s, precision)
+        alone.setPreconditioner(preconditioner)
+        a = alone.project(s.dt, cap, 1e-6, relative_tolerance=1e-6)
+        assert a.iterations == r.iterations and a.solve_status == r.solve_status
+        assert a.residual_l2 == r.residual_l2 and a.max_divergence == r.max_divergence and a.rhs_l2 == r.rhs_l2
+        x, y = g.download(), alone.download()
+        assert np.array_equal(x.u, y.u) and np.array_equal(x.v, y.v) and np.array_equal(x.pressure, y.pressure)
+        alone.destroy()
+    batch.destroy()
