@@ -336,14 +336,15 @@ template <int NT, int WRITERS = 1>
 __device__ bool arrive_count(const GridDesc& g, int run_tiles, int tiles, double4* total, int max_mask)
 {
     __shared__ int is_last;
-    if (threadIdx.x < 32)
+    if (WRITERS > 1 && threadIdx.x < 32)
     {
         if (threadIdx.x < WRITERS)
-            __threadfence(); // the partials before the count
+            __threadfence();
         __syncwarp();
     }
     if (threadIdx.x == 0)
     {
+        __threadfence(); // the partials before the count
         const unsigned int ticket = atomicAdd(g.counter, unsigned(run_tiles));
         is_last = ticket + unsigned(run_tiles) == unsigned(tiles);
     }

@@ -737,6 +737,55 @@ template <typename T> __device__ __forceinline__ UpdateArgs<T> update_args(const
         static_cast<T*>(g.r), g.p, quads, (quads + g.vec_tiles - 1) / g.vec_tiles};
 }
 
+// One quad of a thread's step: its loads, then the update with its sums.
+template <typename T> struct UpdateQuad
+{
+    typename Quad<T>::type d, d0, q, r;
+    double4 p;
+
+    __device__ __forceinline__ void load(const UpdateArgs<T>& a, int j, bool update_p, bool pending)
+    {
+        using Q = typename Quad<T>::type;
+        q = reinterpret_cast<const Q*>(a.q)[j];
+        r = reinterpret_cast<const Q*>(a.r)[j];
+        if (update_p)
+        {
+            d = reinterpret_cast<const Q*>(a.d)[j];
+            p = reinterpret_cast<const double4*>(a.p)[j];
+            if (pending)
+                d0 = reinterpret_cast<const Q*>(a.d0)[j];
+        }
+    }
+
+    __device__ __forceinline__ void apply(const UpdateArgs<T>& a, int j, bool update_p, bool pending, double alpha,
+        double alpha0, double& sum, double& mx, double& sq) const
+    {
+        using Q = typename Quad<T>::type;
+        if (update_p)
+        {
+            double4 pp = p;
+            if (pending)
+                add_step<T>(pp, alpha0, d0);
+            add_step<T>(pp, alpha, d);
+            reinterpret_cast<double4*>(a.p)[j] = pp;
+        }
+        Q rr;
+        rr.x = T(double(r.x) - alpha * double(q.x));
+        rr.y = T(double(r.y) - alpha * double(q.y));
+        rr.z = T(double(r.z) - alpha * double(q.z));
+        rr.w = T(double(r.w) - alpha * double(q.w));
+        reinterpret_cast<Q*>(a.r)[j] = rr;
+        const double e[4] = {double(rr.x), double(rr.y), double(rr.z), double(rr.w)};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+        {
+            sum += e[c];
+            mx = fmax(mx, fabs(e[c]));
+            sq += e[c] * e[c];
+        }
+    }
+};
+
 // GROUP short tiles an entry (kGroup in a crowded plan, see vec_cells): an entry's slices are then
 // worked two at a time, so that both have their loads in flight (a slice of a short tile is about one
 // quad a thread), and folded behind one barrier. A slice's sums are formed alike either way.
@@ -744,13 +793,9 @@ template <typename T, int GROUP>
 __global__ void __launch_bounds__(kVecThreads, kUpdateCtasPerSm)
     k_update(const GridDesc* __restrict__ grids, const Tile* __restrict__ tiles, int count, int parity)
 {
-    using Q = typename Quad<T>::type;
     // Quads per thread and step (FP64 takes one: its quads are twice the registers). A thread
     // visits the same quads in the same order either way.
     constexpr int U = sizeof(T) == 4 ? 2 : 1;
-    // Slices worked at a time, quads of each, and the distance of a thread's quads in a slice.
-    constexpr int SLICES = GROUP == 1 ? 1 : U;
-    constexpr int STEP = kVecThreads * (U / SLICES);
     allow_dependents();
     // The first slice's entry and descriptor fields are read before the wait.
     int i = blockIdx.x;
@@ -772,102 +817,68 @@ __global__ void __launch_bounds__(kVecThreads, kUpdateCtasPerSm)
         SolveState& s = *a.state;
         if (s.done)
             continue;
-        const T* const d = a.d;
-        const T* const q = a.q;
-        T* const r = a.r;
         const double alpha = s.rz / s.dq;
         // Second of a pair: the first's pending step (its direction is the other buffer).
         const bool update_p = parity == 1;
         const bool pending = update_p && s.p_pending;
         const double alpha0 = s.alpha_pending;
-        const T* const d0 = a.d0;
-        const int slices = sum_tiles<GROUP>(g, t), stride = GROUP == 1 ? 0 : sum_tile_stride(g);
-        double4 part;
-#pragma unroll 1
-        for (int k0 = 0; k0 < slices; k0 += SLICES)
-        {
-            int first[SLICES], last[SLICES];
-            double sum[SLICES], mx[SLICES], sq[SLICES];
-#pragma unroll
-            for (int k = 0; k < SLICES; ++k)
-            {
-                first[k] = min(a.quads, a.per * (t.index + (k0 + k) * stride));
-                last[k] = k0 + k < slices ? min(a.quads, first[k] + a.per) : first[k];
-                sum[k] = mx[k] = sq[k] = 0.0;
-            }
-            const int longest = GROUP == 1 ? last[0] - first[0] : a.per;
-            for (int base = int(threadIdx.x); base < longest; base += STEP)
-            {
-                Q dv[U], d0v[U], qv[U], rv[U];
-                double4 pv[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                {
-                    const int k = u % SLICES;
-                    const int j = first[k] + base + u / SLICES * kVecThreads;
-                    if (j < last[k])
-                    {
-                        qv[u] = reinterpret_cast<const Q*>(q)[j];
-                        rv[u] = reinterpret_cast<const Q*>(r)[j];
-                        if (update_p)
-                        {
-                            dv[u] = reinterpret_cast<const Q*>(d)[j];
-                            pv[u] = reinterpret_cast<const double4*>(a.p)[j];
-                            if (pending)
-                                d0v[u] = reinterpret_cast<const Q*>(d0)[j];
-                        }
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                {
-                    const int k = u % SLICES;
-                    const int j = first[k] + base + u / SLICES * kVecThreads;
-                    if (j >= last[k])
-                        continue;
-                    if (update_p)
-                    {
-                        double4 pp = pv[u];
-                        if (pending)
-                            add_step<T>(pp, alpha0, d0v[u]);
-                        add_step<T>(pp, alpha, dv[u]);
-                        reinterpret_cast<double4*>(a.p)[j] = pp;
-                    }
-                    Q rr;
-                    rr.x = T(double(rv[u].x) - alpha * double(qv[u].x));
-                    rr.y = T(double(rv[u].y) - alpha * double(qv[u].y));
-                    rr.z = T(double(rv[u].z) - alpha * double(qv[u].z));
-                    rr.w = T(double(rv[u].w) - alpha * double(qv[u].w));
-                    reinterpret_cast<Q*>(r)[j] = rr;
-                    const double e[4] = {double(rr.x), double(rr.y), double(rr.z), double(rr.w)};
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                    {
-                        sum[k] += e[c];
-                        mx[k] = fmax(mx[k], fabs(e[c]));
-                        sq[k] += e[c] * e[c];
-                    }
-                }
-            }
-            if constexpr (GROUP == 1)
-                part = block_reduce4<kVecThreads>(make_double4(sum[0], mx[0], sq[0], 0), 2);
-            else
-            {
-#pragma unroll
-                for (int k = 0; k < SLICES; ++k)
-                    if (k0 + k < slices)
-                        reduce_to_slot<3>(slots[flip][k0 + k], make_double4(sum[k], mx[k], sq[k], 0), 2);
-            }
-        }
         if constexpr (GROUP == 1)
         {
+            const int first = min(a.quads, a.per * t.index);
+            const int last = min(a.quads, first + a.per);
+            double sum = 0.0, mx = 0.0, sq = 0.0;
+            for (int base = first + int(threadIdx.x); base < last; base += kVecThreads * U)
+            {
+                UpdateQuad<T> x[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (base + u * kVecThreads < last)
+                        x[u].load(a, base + u * kVecThreads, update_p, pending);
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (base + u * kVecThreads < last)
+                        x[u].apply(a, base + u * kVecThreads, update_p, pending, alpha, alpha0, sum, mx, sq);
+            }
+            const double4 part = block_reduce4<kVecThreads>(make_double4(sum, mx, sq, 0), 2);
             if (threadIdx.x == 0)
                 g.partial[t.index] = part;
+            ++run;
         }
         else
-            write_partials<kVecThreads, GROUP>(g, t, slots[flip], 2);
-        flip ^= 1;
-        run += slices;
+        {
+            const int slices = sum_tiles<GROUP>(g, t), stride = sum_tile_stride(g);
+#pragma unroll 1
+            for (int k0 = 0; k0 < slices; k0 += U)
+            {
+                int first[U], last[U];
+                double sum[U], mx[U], sq[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                {
+                    first[u] = min(a.quads, a.per * (t.index + (k0 + u) * stride));
+                    last[u] = k0 + u < slices ? min(a.quads, first[u] + a.per) : first[u];
+                    sum[u] = mx[u] = sq[u] = 0.0;
+                }
+                for (int base = int(threadIdx.x); base < a.per; base += kVecThreads)
+                {
+                    UpdateQuad<T> x[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        if (first[u] + base < last[u])
+                            x[u].load(a, first[u] + base, update_p, pending);
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        if (first[u] + base < last[u])
+                            x[u].apply(a, first[u] + base, update_p, pending, alpha, alpha0, sum[u], mx[u], sq[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (k0 + u < slices)
+                        reduce_to_slot<3>(slots[flip][k0 + u], make_double4(sum[u], mx[u], sq[u], 0), 2);
+            }
+            run += write_partials<kVecThreads, GROUP>(g, t, slots[flip], 2);
+            flip ^= 1;
+        }
         const int next = i + gridDim.x;
         if (next >= count || tiles[next].grid != t.grid)
         {

@@ -146,6 +146,9 @@ struct TailMeans
 // Dynamic shared memory: the coarsest inverse, its right-hand side in FP64, the table's header, and
 // the levels' elements (at most 10840 in FP32 and 5912 in FP64 over every level shape a tail
 // takes). Everything is addressed by element offsets, so that every access is a shared-memory one.
+// Every launch has the largest table's (its registers leave room for one CTA an SM anyway), so no table
+// outgrows a launch; asking for a table's own and checking it in the kernel delayed the copies by
+// 0.3 us.
 constexpr size_t kTailSolveBytes = kTailInverseBytes + kMaxCoarse * sizeof(double);
 inline size_t tail_bytes(int elements, size_t elem) { return kTailSolveBytes + kTailHeader + size_t(elements) * elem; }
 constexpr size_t kTailMaxBytes = kTailSolveBytes + kTailHeader + 5912 * sizeof(double);
@@ -341,7 +344,17 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
     // plain loads for the set-up, and with the tables and the coarsest inverse by bulk copy for the
     // cycle.
     const int smoothed = table->smoothed, first = table->first, tables = table->tables, zeroed = table->zeroed;
-    const int elements = table->elements;
+    // Bulk copies write 16-byte aligned shared addresses only: a misplaced buffer is reported.
+    const bool aligned = (smem_address(tail_smem) & 15u) == 0;
+    if (threadIdx.x == 0 && aligned)
+    {
+        mbarrier_init(&bar, 1);
+        fence_async_shared();
+        const unsigned bytes = kTailHeader + unsigned(tables) * sizeof(T);
+        mbarrier_expect_tx(&bar, bytes + unsigned(kTailInverseBytes));
+        bulk_load(tail_smem + kTailSolveBytes, table, bytes, &bar);
+        bulk_load(inverse, g.coarse_inverse, unsigned(kTailInverseBytes), &bar);
+    }
     // This warp's level (-1: none).
     int role = -1, level_warp = warp, warps_needed = 0;
 #pragma unroll
@@ -356,19 +369,6 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
             else
                 level_warp -= warps;
         }
-    }
-    // Bulk copies write 16-byte aligned shared addresses only, and a level's barrier waits for all its
-    // warps: a misplaced buffer or a table that this launch is too small for is reported.
-    const bool ready = (smem_address(tail_smem) & 15u) == 0 && 32 * warps_needed <= kThreads &&
-        unsigned(kTailSolveBytes) + kTailHeader + unsigned(elements) * sizeof(T) <= dynamic_smem_bytes();
-    if (threadIdx.x == 0 && ready)
-    {
-        mbarrier_init(&bar, 1);
-        fence_async_shared();
-        const unsigned bytes = kTailHeader + unsigned(tables) * sizeof(T);
-        mbarrier_expect_tx(&bar, bytes + unsigned(kTailInverseBytes));
-        bulk_load(tail_smem + kTailSolveBytes, table, bytes, &bar);
-        bulk_load(inverse, g.coarse_inverse, unsigned(kTailInverseBytes), &bar);
     }
     const TailPlace& place = table->place[max(role, 0)];
     const int S = place.S;
@@ -417,15 +417,13 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
     const T* const rhs = static_cast<const T*>(table->rhs);
     T* const out = static_cast<T*>(table->out);
     // Edges and lines start at zero: what lies outside a level is never written.
-    if (ready)
-    {
-        for (int i = threadIdx.x; i < zeroed; i += blockDim.x)
-            m[tables + i] = T(0);
-        if (threadIdx.x < kMaxCoarse)
-            coarse_rhs[threadIdx.x] = 0.0;
-    }
+    for (int i = threadIdx.x; i < zeroed; i += blockDim.x)
+        m[tables + i] = T(0);
+    if (threadIdx.x < kMaxCoarse)
+        coarse_rhs[threadIdx.x] = 0.0;
     __syncthreads();
-    if (stage_failed(ready && mbarrier_wait(&bar, 0), g.state))
+    // A level's barrier waits for all its warps, so they must be in this launch.
+    if (stage_failed(aligned && mbarrier_wait(&bar, 0) && 32 * warps_needed <= kThreads, g.state))
         return;
     const TailPlace& own = shared_table.place[max(role, 0)];
     const TailPlace& finer = shared_table.place[max(role - 1, 0)];
@@ -486,7 +484,7 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
         if (int(threadIdx.x) < cells)
             coarse_rhs[threadIdx.x] = double(value);
         __syncthreads();
-        if (means)
+        if (__builtin_expect(means, 0))
         {
             for (int i = lane; i < cells; i += 32)
                 mean += inverse[TailMeans::open(i)] * coarse_rhs[i];

@@ -17,14 +17,6 @@ __device__ __forceinline__ uint32_t smem_address(const void* p)
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// Dynamic shared memory of this launch, in bytes.
-__device__ __forceinline__ uint32_t dynamic_smem_bytes()
-{
-    uint32_t bytes;
-    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(bytes));
-    return bytes;
-}
-
 __device__ __forceinline__ void mbarrier_init(uint64_t* bar, unsigned count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_address(bar)), "r"(count) : "memory");
