@@ -334,6 +334,7 @@ struct Grid
 
     std::vector<HostLevel> levels;
     int tail = 0;
+    size_t tail_smem = 0;
     int tail_threads = 0;
     int tail_cells = 1024; // largest level the one-CTA tail takes (autotuned)
 
@@ -458,7 +459,8 @@ void choose_tail(Grid& g)
     for (int i = 0; i < t.smoothed; ++i)
         warps += t.place[i].warps;
     g.tail_threads = 32 * warps;
-    if (tail_bytes(t.elements, g.elem) > kTailMaxBytes || kTailHeader + t.tables * g.elem > kTailTableBytes ||
+    g.tail_smem = tail_bytes(t.elements, g.elem);
+    if (g.tail_smem > kTailMaxBytes || kTailHeader + t.tables * g.elem > kTailTableBytes ||
         g.tail_threads > (g.elem == 4 ? kTailWideThreads : kTailThreads<double>))
         fail(FC_ERR_CUDA, "coarse tail of a %dx%d grid does not fit one CTA", g.W, g.H);
 }
@@ -1080,6 +1082,7 @@ struct Plan
     int max_levels = 0;
     int max_tail = 0;
     int cells_max[kMaxLevels] = {}; // most cells of any grid's level, per level
+    size_t tail_smem = 0;
     int tail_threads = 0;
     // First tail level of each grid when the plan was made: the tiles and the tail's launch follow
     // from it, so a plan is remade once a grid's tail moves (plan_current).
@@ -1225,6 +1228,7 @@ std::unique_ptr<Plan> make_plan(const std::vector<Grid*>& grids, cudaStream_t st
     {
         plan->max_levels = std::max(plan->max_levels, int(g->levels.size()));
         plan->max_tail = std::max(plan->max_tail, g->tail);
+        plan->tail_smem = std::max(plan->tail_smem, g->tail_smem);
         plan->tail_threads = std::max(plan->tail_threads, g->tail_threads);
         plan->tails.push_back(g->tail);
         for (size_t l = 0; l < g->levels.size(); ++l)
@@ -1403,9 +1407,9 @@ template <typename T, int kThreads> void launch_tail_kernel(Plan& p, bool depend
     static SharedOptIn opt_in;
     opt_in(kernel, kTailMaxBytes, "tail shared memory");
     if (dependent)
-        FC_LAUNCH_DEP(kernel, p.n(), kThreads, kTailMaxBytes, s, p.d_desc);
+        FC_LAUNCH_DEP(kernel, p.n(), kThreads, p.tail_smem, s, p.d_desc);
     else
-        FC_LAUNCH(kernel, p.n(), kThreads, kTailMaxBytes, s, p.d_desc);
+        FC_LAUNCH(kernel, p.n(), kThreads, p.tail_smem, s, p.d_desc);
 }
 
 template <typename T> void launch_tail(Plan& p, bool dependent, cudaStream_t s)
