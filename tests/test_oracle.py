@@ -173,6 +173,7 @@ def test_restatement_large_mixed_pressure_within_default_budget(oracle):
     assert r.converged and r.max_divergence <= 1e-6
 
 
+@needs_reference
 def test_restatement_matches_live_reference_on_odd_grid(oracle):
     """FluidGridTests.cpp:683-708's 513x257 grid: the restatement and the reference engine itself
     agree within the reference test's 2e-7."""
