@@ -829,7 +829,14 @@ def main():
         print(f"bench.py: --gpus {args.gpus} but WORLD_SIZE is {world}", file=sys.stderr)
         sys.exit(2)
     if args.impl == "reference":
-        line = run_reference(args, world, rank)
+        from oracle import oracle
+
+        if oracle.reference_available():
+            line = run_reference(args, world, rank)
+        else:
+            # The arm drives the reference's own engine or nothing: the restatement is not it.
+            line = {"impl": "reference", "unavailable": "the reference engine (oracle/_ref) is not built: no reference sources"}
+            line = line if rank == 0 else None
         if line is not None:
             print(json.dumps(line), flush=True)
         return

@@ -56,6 +56,21 @@ def test_reference_arm_line_keeps_integer_steps_and_the_shared_config(monkeypatc
     assert bench.run_reference(args, 2, 1) is None  # other ranks do no work
 
 
+def test_reference_arm_without_the_engine_says_so_and_times_nothing(monkeypatch, capsys):
+    import json
+
+    from oracle import oracle
+
+    bench = _bench()
+    monkeypatch.setattr(oracle, "reference_available", lambda: False)
+    monkeypatch.setattr(bench, "run_reference", None)  # not called
+    monkeypatch.delenv("WORLD_SIZE", raising=False)
+    monkeypatch.setattr(bench.sys, "argv", ["bench.py", "--impl", "reference"])
+    bench.main()
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and "not built" in line["unavailable"] and set(line) == {"impl", "unavailable"}
+
+
 def test_cuda_arm_never_overwrites_the_step_count():
     """`steps` is the timed step count; every leg sits under its own key."""
     import ast
