@@ -181,7 +181,7 @@ struct GridDesc
     // p = 0, neither solid nor liquid phase (f > 0.5). Written by k_coefficients from `fraction`.
     unsigned char* air;
     const double* fraction;  // liquid fraction, W x H, unpadded
-    double* density;         // W x H, unpadded
+    double* density;         // W x H, unpadded: scratch of transport (PLIC fills it with densities)
     double* const* masses;   // device array of `components` W x H mass fields
     int components;
     const void* maps;        // TMA tensor maps of the smoothed levels (see fc_stage.cuh)

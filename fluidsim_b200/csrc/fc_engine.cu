@@ -1894,8 +1894,9 @@ void advect_semi_lagrangian(Grid& g, double dt, bool wait)
         // The new velocities first: the cell fields trace through the old ones until the commit.
         FC_LAUNCH(k_advect_velocity<T>, p.faces.count, kVecThreads, 0, s, p.d_desc, p.at(p.faces), scale, half,
             static_cast<T*>(g.u_next), static_cast<T*>(g.v_next));
-        // Scratch for the new cell fields: the upload staging, and the density and right-hand side,
-        // which every projection (and PLIC transport) forms anew before it reads them.
+        // Scratch for the new cell fields: the upload staging, the right-hand side, which every
+        // projection forms anew, and the density array, which PLIC transport alone uses, filling it
+        // itself (a projection reads the component masses).
         double* const scratch[kAdvectFields] = {g.staging, g.desc.density, g.desc.b};
         const int fields = 1 + g.components();
         for (int first = 0; first < fields; first += kAdvectFields)
@@ -2127,9 +2128,9 @@ size_t viscosity_layout(const Grid& g, ViscWork* work, char* base)
     return total;
 }
 
-// First level of the one-CTA tail: the first whose levels fit 200 KB of shared memory together (in
-// FP32 4,300 nodes, so a first level of up to 3,200, e.g. 56 x 56). At 4096 x 4096 it takes the levels
-// from 32 x 32 on.
+// First level of the one-CTA tail: the first whose levels fit 200 KB of shared memory together (4,266
+// nodes in FP32 and 2,133 in FP64: the largest square first levels are 55 x 55 and 38 x 38). At
+// 4096 x 4096 it takes the levels from 32 x 32 on.
 size_t viscosity_tail(const ViscWork& w, size_t elem)
 {
     size_t first = w.lev.size() - 1, bytes = 0;
@@ -2551,7 +2552,7 @@ double time_kernel(Grid& g, int kernel, int repeats)
 // Autotuning of the multigrid schedule
 // ------------------------------------------------------------------------------------------
 //
-// The tail threshold (the largest level the one-CTA tail cycles in shared memory; the levels
+// The tail threshold (the largest level the one-CTA tail cycles in registers; the levels
 // above it run the strip kernels) changes which kernels run, not the arithmetic: both apply
 // the same red-black sweeps, transfers and coarsest solve. The tuner times V-cycles of a plan
 // under each candidate and keeps the fastest.

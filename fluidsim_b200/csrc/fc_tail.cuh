@@ -57,7 +57,7 @@ template <typename T> constexpr int kTailPlane = (sizeof(T) == 4 ? 18 : 10) * 32
 struct TailPlace
 {
     int w, h, S, lanes, warps;
-    int rows, cols, px, py, edges, lines, sol, sol_stride, unused;
+    int rows, cols, px, py, edges, lines, sol, sol_stride;
     const void* right;
     const void* down;
     const void* inv;
@@ -68,7 +68,7 @@ struct TailPlace
 // kTailHeader on the transfer weights (`tables` elements, at the offsets in `place`).
 struct TailTable
 {
-    int smoothed, first, cells, tables;
+    int smoothed, first, tables;
     int zeroed;   // elements of edges and lines, which start at zero, behind the tables
     int elements; // all elements
     const void* rhs; // right-hand side and solution of the first level
@@ -124,7 +124,6 @@ inline void tail_layout(TailTable& t, int plane)
         p.sol = take(p.sol_stride * p.h);
     }
     t.elements = cursor;
-    t.cells = t.place[t.smoothed].w * t.place[t.smoothed].h;
 }
 
 // The coarsest inverse's rows are 72 doubles apart, in global and in shared memory: the four rows

@@ -13,7 +13,8 @@
 // right-hand side, the residual is restricted where it is formed (k_visc_restrict), the prolongation
 // is swept where it is formed (k_visc_prolong_smooth), and the small levels run in one CTA
 // (k_visc_tail): 17 launches a CG iteration instead of 41 at 321 x 239. Measured, whole solves in
-// FP32 before and after: 321 x 239 6.65 -> 5.69 ms, 4096 x 4096 189 -> 159 ms.
+// FP32 from one pass per step of the method to this form, on one box: 321 x 239 6.72 -> 4.42 ms,
+// 4096 x 4096 189 -> 164 ms.
 //
 // Layout: the (w+1) x (h+1) node lattice of a level, row-major; node p holds u face p (x) and v
 // face p (y) as one 2-vector, and 4 coefficients (cell mu, vertex mu, u-face mass, v-face mass).

@@ -355,7 +355,7 @@ int fc_batch_project(fc_batch* batch, const double* dts, int max_iterations, dou
 int fc_batch_get_stream(const fc_batch* batch, void** stream);
 
 /* Autotuning of the multigrid schedule (no reference counterpart). The tail threshold is the
- * largest level the one-block tail cycles in shared memory; larger levels run the strip
+ * largest level the one-block tail cycles in registers; larger levels run the strip
  * kernels. It changes which kernels run, not the arithmetic. fc_autotune and fc_batch_autotune
  * time `repeats` V-cycles of the grid's (or the batch's) plan under each candidate threshold
  * (256, 1024, 4096 cells) and keep the fastest; the grids' states are left as they were.

@@ -9,9 +9,11 @@ from fluidsim_b200._native import FluidCudaError
 pytestmark = pytest.mark.gpu
 
 # A single level, thin lattices, the restriction's and prolongation's 32 x 8 tiles and their
-# remainders, levels of at most and of more than one node per thread of the one-CTA cycle, and two
-# and three levels above it.
-SIZES = [(8, 8), (3, 90), (90, 3), (31, 31), (32, 33), (63, 16), (66, 65), (97, 130), (257, 66), (300, 211)]
+# remainders, levels of at most and of more than one node per thread of the one-CTA cycle, the largest
+# squares that are all in it and the next ones (55 and 56 in FP32, 38 and 39 in FP64), and two and
+# three levels above it.
+SIZES = [(8, 8), (3, 90), (90, 3), (31, 31), (32, 33), (63, 16), (55, 55), (56, 56), (38, 38),
+         (39, 39), (66, 65), (97, 130), (257, 66), (300, 211)]
 
 
 @pytest.mark.parametrize("precision,bound", [("fp64", 1e-10), ("fp32", 1e-3)])
