@@ -322,6 +322,56 @@ __device__ __forceinline__ void tail_prolong(Strip<T, kTailK>& s, const TailLane
     }
 }
 
+// One thread's share of a product with a row of the coarsest inverse, and the sum of the eight.
+__device__ __forceinline__ double coarse_dot(const double* row, const double* rhs, int part)
+{
+    const double* a = row + part;
+    double z = 0.0, z1 = 0.0;
+#pragma unroll
+    for (int i = 0; i < kMaxCoarse / 16; ++i)
+    {
+        z += a[16 * i] * rhs[part + 16 * i];
+        z1 += a[16 * i + 8] * rhs[part + 16 * i + 8];
+    }
+    return z + z1;
+}
+
+__device__ __forceinline__ double eight_lane_sum(double z)
+{
+    z += __shfl_xor_sync(0xffffffffu, z, 1);
+    z += __shfl_xor_sync(0xffffffffu, z, 2);
+    return z + __shfl_xor_sync(0xffffffffu, z, 4);
+}
+
+// The coarsest solve with an inverse that has no means folded in (k_rebuild_tail): the mean comes off
+// the right-hand side in `rhs`, and the solution's, from the row of the column sums, off the solution.
+// Returns the right-hand side's mean. Rare, and kept out of the cycle's code: inlined it cost every
+// V-cycle 0.2 us.
+template <typename T, int kThreads>
+__device__ __noinline__ double tail_solve_means(const double* inverse, double* rhs, double share, int cells, int sol)
+{
+    double mean = 0.0;
+    for (int i = threadIdx.x & 31; i < cells; i += 32)
+        mean += inverse[TailMeans::open(i)] * rhs[i];
+    mean = warp_sum(mean) * share;
+    __syncthreads();
+    if (int(threadIdx.x) < cells)
+        rhs[threadIdx.x] -= mean;
+    __syncthreads();
+    const int part = threadIdx.x & 7;
+    const double gauge = eight_lane_sum(coarse_dot(inverse + TailMeans::sums(0), rhs, part)) * share;
+    T* const m = tail_elements<T>();
+    for (int base = 0; base < kMaxCoarse; base += kThreads / 8)
+    {
+        const int row = base + int(threadIdx.x >> 3);
+        const double z = eight_lane_sum(coarse_dot(inverse + min(row, kMaxCoarse - 1) * kTailInverseStride, rhs, part));
+        if (row < cells && part == 0)
+            m[sol + row] = inverse[TailMeans::open(row)] != 0.0 ? T(z - gauge) : T(0);
+    }
+    __syncthreads();
+    return mean;
+}
+
 template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) k_mg_tail(const GridDesc* __restrict__ grids)
 {
     using P = typename Pair<T>::type;
@@ -454,56 +504,31 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
         return;
 
     // The coarsest level (at most 64 cells): mean-free, explicit inverse, mean-zero gauge
-    // (PressureMultigrid.cpp:347-384), its solution to last.sol. Eight threads per row, each with every
-    // eighth entry in two chains. With the means folded into the inverse that is one product; otherwise
-    // the right-hand side's mean comes off first (and is returned), and the solution's from the row of
-    // the column sums.
+    // (PressureMultigrid.cpp:347-384), its solution to last.sol: one product with the means folded
+    // into the inverse, or a solve that takes them itself (tail_solve_means) and returns the
+    // right-hand side's. Eight threads per row, each with every eighth entry in two chains.
     auto solve_coarsest = [&](T value)
     {
-        const double share = inverse[TailMeans::share];
-        const bool means = share != 0.0;
-        const int part = threadIdx.x & 7;
-        double mean = 0.0, gauge = 0.0;
-        auto product = [&](const double* row)
-        {
-            const double* a = row + part;
-            double z = 0.0, z1 = 0.0;
-#pragma unroll
-            for (int i = 0; i < kMaxCoarse / 16; ++i)
-            {
-                z += a[16 * i] * coarse_rhs[part + 16 * i];
-                z1 += a[16 * i + 8] * coarse_rhs[part + 16 * i + 8];
-            }
-            z += z1;
-            z += __shfl_xor_sync(0xffffffffu, z, 1);
-            z += __shfl_xor_sync(0xffffffffu, z, 2);
-            z += __shfl_xor_sync(0xffffffffu, z, 4);
-            return z;
-        };
         if (int(threadIdx.x) < cells)
             coarse_rhs[threadIdx.x] = double(value);
         __syncthreads();
-        if (__builtin_expect(means, 0))
-        {
-            for (int i = lane; i < cells; i += 32)
-                mean += inverse[TailMeans::open(i)] * coarse_rhs[i];
-            mean = warp_sum(mean) * share;
-            __syncthreads();
-            if (int(threadIdx.x) < cells)
-                coarse_rhs[threadIdx.x] -= mean;
-            __syncthreads();
-            gauge = product(inverse + TailMeans::sums(0)) * share;
-        }
+        const double share = inverse[TailMeans::share];
+        if (__builtin_expect(share != 0.0, 0))
+            return tail_solve_means<T, kThreads>(inverse, coarse_rhs, share, cells, last.sol);
+        const int part = threadIdx.x & 7;
 #pragma unroll
         for (int base = 0; base < kMaxCoarse; base += kThreads / 8)
         {
             const int row = base + int(threadIdx.x >> 3);
-            const double z = product(inverse + min(row, kMaxCoarse - 1) * kTailInverseStride);
+            double z = 0.0;
+            if (row < kMaxCoarse)
+                z = coarse_dot(inverse + row * kTailInverseStride, coarse_rhs, part);
+            z = eight_lane_sum(z);
             if (row < cells && part == 0)
-                m[last.sol + row] = means && inverse[TailMeans::open(row)] == 0.0 ? T(0) : T(z - gauge);
+                m[last.sol + row] = T(z);
         }
         __syncthreads();
-        return mean;
+        return 0.0;
     };
     if (smoothed == 0)
     {
@@ -683,7 +708,7 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
 // differently from the column loop.) Rounding moves either method's pivots by at most a few times
 // 64 epsilon of the largest diagonal (the Schur complements of this diagonally dominant matrix do not
 // grow), so above the limit both accept. Densities of 1000 : 1 leave pivots of 1e-5 and more.
-// The whole kernel on a 64 x 64 grid in FP32: 41 us, 98 us where a wall across it needs the column loop.
+// The whole kernel on a 64 x 64 grid in FP32: 40 us, 101 us where a wall across it needs the column loop.
 constexpr double kSealedPivot = 1.0 / (1 << 24);
 
 // Eight threads hold a row in registers (every eighth column).
@@ -696,17 +721,19 @@ struct CoarseRow
 };
 
 // The inverse of the operator in `row` by its Cholesky factor, in the place of the operator; true
-// if a pivot is not positive or not finite. `unknowns` has the bits of the unknowns' cells.
+// if a pivot is not positive or not finite. `unknowns` has the bits of the unknowns' cells, and
+// `factor` is global scratch of a row of kTailInverseStride a cell (in shared memory it made every
+// rebuild's launch larger).
 //
 // The factor L is formed right-looking: every entry takes the reference's subtractions in the
 // reference's order (PressureMultigrid.cpp:313-339), each product fused into its subtraction. Y = L^-1
 // takes the place of the columns L is done with, and the inverse is Y^T Y. Step k publishes one
 // vector: column k of L below the diagonal, and row k of Y up to it. Every warp carries the diagonal,
 // two entries a lane, so its next pivot needs no other warp: one barrier a step, double-buffered.
-static __device__ __noinline__ bool invert_factor(CoarseRow& row, const double* diagonal, unsigned long long unknowns, int cells)
+static __device__ __noinline__ bool invert_factor(CoarseRow& row, const double* diagonal, unsigned long long unknowns, int cells,
+    double* factor)
 {
     constexpr int N = kMaxCoarse, E = kCoarseColumns;
-    __shared__ double factor[N * kTailInverseStride];
     __shared__ double step[2][N];
     __shared__ int failed;
     const int r = row.r, part = row.part, lane = threadIdx.x & 31;
@@ -779,16 +806,18 @@ static __device__ __noinline__ bool invert_factor(CoarseRow& row, const double* 
         factor[r * kTailInverseStride + c] = mine && c <= r && (unknowns >> c & 1) ? a[i] : 0.0;
         a[i] = 0.0;
     }
+    __threadfence_block();
     __syncthreads();
     // Entry (r, c) sums Y[k][r] Y[k][c] over k >= max(r, c): the terms before it are zero.
     for (int k = first_row; k < cells; ++k)
     {
         const double* const y = factor + k * kTailInverseStride;
-        const double yr = y[r];
+        const double yr = __ldcg(y + r);
 #pragma unroll
         for (int i = 0; i < E; ++i)
-            a[i] = fma(yr, y[part + 8 * i], a[i]);
+            a[i] = fma(yr, __ldcg(y + part + 8 * i), a[i]);
     }
+    __syncthreads(); // the caller writes there
 #pragma unroll
     for (int i = 0; i < E; ++i)
         row.a[i] = a[i];
@@ -920,7 +949,7 @@ template <typename T> __global__ void __launch_bounds__(kCoarseThreads, 1) k_reb
 #pragma unroll
         for (int i = 0; i < E; ++i)
             row.a[i] = a[i];
-        failed = invert_factor(row, diagonal, unknowns, cells);
+        failed = invert_factor(row, diagonal, unknowns, cells, g.coarse_inverse);
 #pragma unroll
         for (int i = 0; i < E; ++i)
             a[i] = row.a[i];
