@@ -704,7 +704,7 @@ template <typename T, int kThreads> __global__ void __launch_bounds__(kThreads) 
 // a rounding error, whose sign decides between breakdown and solve, and the inverse has entries of
 // 1e16, in which folded means would drown every other part's. So if a pivot is not above kSealedPivot
 // of the largest diagonal, the factor is formed again by the reference's column loop (invert_factor)
-// and the means are left to the solve. (Gauss-Jordan pivots decided 26 of 96 sealed 8 x 8 scenes
+// and the means are left to the solve. (Gauss-Jordan pivots decided 26 of 96 sealed 8 x 8 and 7 x 9 scenes
 // differently from the column loop.) Rounding moves either method's pivots by at most a few times
 // 64 epsilon of the largest diagonal (the Schur complements of this diagonally dominant matrix do not
 // grow), so above the limit both accept. Densities of 1000 : 1 leave pivots of 1e-5 and more.
